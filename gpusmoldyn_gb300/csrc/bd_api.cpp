@@ -129,7 +129,8 @@ struct bd_system {
   DevBuf<float4> state0, state1, scatter, bins;
   cudaMemPool_t pool = nullptr;  // stream-ordered scratch of host transfers (keeps its memory)
   DevBuf<unsigned long long> best;
-  DevBuf<uint32_t> cell_count, cell_start, tile_sums, big;
+  DevBuf<uint32_t> cell_count, cell_start, tile_sums;
+  DevBuf<uint2> big;
   DevBuf<uint4> match_list;
   DevBuf<float4> big_scratch;  // allocated when a cell first outgrows the pair kernel
   DevBuf<DevPair> pairs;
@@ -188,7 +189,7 @@ KParams make_params(bd_system* h) {
   p.big = h->big.p;
   p.big_scratch = h->big_scratch.p;
   p.big_cap = (uint32_t)h->big.n;
-  p.big_scratch_cap = (uint32_t)h->big_scratch.n;
+  p.big_scratch_cap = h->big_scratch.n;
   p.ctrl = h->ctrl.p;
   p.inst = h->dinst.p;
   if (!h->hinst.empty()) p.inst0 = h->hinst[0];
@@ -444,7 +445,7 @@ bd_status grow_particles(bd_system* h, uint64_t cap) {
   if (!h->panels.empty()) BD_CUDA(h->surf_queue.alloc(cap));
   // cells above 128 records (the large-cell kernel's queue) number at most cap / 129
   BD_CUDA(h->big.alloc(cap / 129 + 2));
-  if (h->big_scratch.n) BD_CUDA(h->big_scratch.alloc(cap));
+  if (h->big_scratch.n) BD_CUDA(h->big_scratch.alloc(2 * cap));
   if (h->have_particles && h->hctrl->n_slots > 0) {
     const float4* src = h->hctrl->cur ? h->state1.p : h->state0.p;
     BD_CUDA(cudaMemcpyAsync(s0.p, src, (size_t)h->hctrl->n_slots * sizeof(float4), cudaMemcpyDeviceToDevice,
@@ -1334,7 +1335,7 @@ BD_API bd_status bd_synchronize(bd_handle h) {
         if (st) return st;
         c.bin_need = 0;
       }
-      if (c.status & kStatScratch) BD_CUDA(h->big_scratch.alloc(h->capacity));
+      if (c.status & kStatScratch) BD_CUDA(h->big_scratch.alloc(2 * h->capacity));
       if (c.status & kStatPairs) {
         uint64_t cap = std::max<uint64_t>(2ull * h->pair_cap, (uint64_t)c.n_pairs + c.n_pairs / 2 + 1024);
         if (cap > 0x7FFFFFFFull) return BD_ERR_CAPACITY;
@@ -1345,7 +1346,8 @@ BD_API bd_status bd_synchronize(bd_handle h) {
       BD_CUDA(cudaMemsetAsync(h->pending.p, 0, h->pending.n * sizeof(unsigned long long), h->stream));
       c.status = 0;
       c.n_pairs = 0;
-      c.n_big = 0;
+      c.big_queue = 0;
+      c.big_max = 0;
       c.n_surf = 0;
       c.surf_ticket = 0;
       c.n_virtual = 0;

@@ -1005,6 +1005,7 @@ __device__ __forceinline__ void emit_pair(const KParams& p, DevCtrl* c, uint32_t
 // Cells with more records than this are handed from k_pairs_cells to
 // k_pairs_big, which gives each of them a whole CTA.
 constexpr uint32_t kBigCell = 128;
+constexpr uint32_t kBigChunk = 2048;  // records of a unit: sorted in one pass through shared memory (16 KiB of keys)
 constexpr int kBigGrid = 304;  // most CTAs of the large-cell kernel (cells they take in turn)
 
 // First record of a cell: its bin, or its range of the compact scatter buffer.
@@ -1357,8 +1358,12 @@ __global__ void __launch_bounds__(256, 4) k_pairs_cells(KParams p) {
         n = __ldg(&p.cell_start[cell + 1]) - cs;
         if (kBinned) p.cell_count[cell] = 0u;
         if (n > kBigCell) {
-          const uint32_t b = atomicAdd(&c->n_big, 1u);
-          if (b < p.big_cap) p.big[b] = cell;
+          // its place in the queue and its first unit in one atomic, so
+          // that the entries are in unit order
+          const unsigned long long b =
+              atomicAdd(&c->big_queue, (unsigned long long)((n + kBigChunk - 1u) / kBigChunk) << 32 | 1ull);
+          atomicMax(&c->big_max, n);
+          if ((uint32_t)b < p.big_cap) p.big[(uint32_t)b] = make_uint2(cell, (uint32_t)(b >> 32));
           else atomicOr(&c->status, kStatBounds);
           n = 0;
         }
@@ -1510,23 +1515,184 @@ __global__ void __launch_bounds__(256, 4) k_pairs_cells(KParams p) {
   if (kHasBim && fq > 0) drain_faces<kBinned, kSingle>(p, c, fqueue, fq, kSingle ? s_maxr : nullptr, adv0);
 }
 
-constexpr uint32_t kBigChunk = 2048;  // records sorted per shared-memory pass
+// ------------------------------------------------------------ large cells
+// A cell of more than kBigCell records (particles released at one point, a
+// collapse) is cut into units of kBigChunk records, and every phase spreads
+// units, not cells, over the CTAs: with a CTA per cell, 20,000 particles
+// released at a point kept one SM busy for 20 to 31 ms a step while 151
+// idled; the same steps take 0.13 ms (half of it sorting, half pairs).
+// What bounds the phases now is latency: the bitonic network's barriers,
+// the dependent L2 loads of the rank searches, the grid barriers between
+// phases.
+constexpr uint32_t kBigWays = 32;     // sorted runs one merge pass joins
+constexpr uint32_t kBigParts = 32;    // most CTAs that share a unit's pair search
+constexpr uint32_t kBigSegments = 8;  // pieces of a seeker block's sweep when few units are queued
 
-// Records in [0, len) of the sorted run `run` that order before `e`
-// (kOrEqual: before or equal).
-template <bool kOrEqual>
-__device__ __forceinline__ uint32_t run_rank(const float4* run, uint32_t len, const float4& e) {
-  uint32_t lo = 0, hi = len;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    const float4 q = run[mid];
-    if (rec_less(q, e) || (kOrEqual && rec_equal(q, e))) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
+// Merge passes that turn a cell of n records, sorted unit by unit, into one
+// run.
+__device__ __forceinline__ uint32_t big_passes(uint32_t n) {
+  uint32_t passes = 0;
+  for (uint64_t w = kBigChunk; w < n; w *= kBigWays) ++passes;
+  return passes;
 }
 
-// CTA-uniform status read (the large-cell kernels use barriers).
+// A queued cell and its records.
+struct BigCell {
+  uint32_t cell, cs, n;
+  uint32_t first;  // first record of the unit asked for
+};
+
+// Queue entry of unit u: entries hold (cell, first unit) in unit order.
+__device__ __forceinline__ BigCell big_unit(const KParams& p, uint32_t nbig, uint32_t u) {
+  uint32_t lo = 0, hi = nbig;
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (__ldcg(&p.big[mid]).y <= u) lo = mid;
+    else hi = mid;
+  }
+  const uint2 e = __ldcg(&p.big[lo]);
+  BigCell b;
+  b.cell = e.x;
+  b.cs = p.cell_start[e.x];
+  b.n = p.cell_start[e.x + 1] - b.cs;
+  b.first = (u - e.y) * kBigChunk;
+  return b;
+}
+
+// The two buffers the merge passes of a cell alternate between: its ranges
+// of the two halves of big_scratch.  (The cell's own bin, free once its
+// units are sorted, made a poor second buffer: the groups of a bin lie
+// n_cells x 64 bytes apart, a page each for a crowded cell, and the
+// searches of the pair phase ran on TLB misses.)
+__device__ __forceinline__ float4* big_buffer(const KParams& p, uint32_t cs, uint32_t which) {
+  return p.big_scratch + (which & 1u ? p.capacity : 0u) + cs;
+}
+
+// Sum over the runs of width w in [lo, hi) of the records that order before
+// e (before or equal in runs ahead of e's own), e's own run excluded.  Eight
+// searches at a time, so that their loads are in flight together.
+__device__ __forceinline__ uint32_t runs_rank(const float4* v, uint32_t w, uint32_t lo, uint32_t hi, uint32_t own,
+                                              const float4& e) {
+  constexpr uint32_t kIlp = 8;
+  const uint32_t runs = (hi - lo + w - 1u) / w;
+  uint32_t rank = 0;
+  for (uint32_t r = 0; r < runs; r += kIlp) {
+    uint32_t at[kIlp], len[kIlp];
+#pragma unroll
+    for (uint32_t k = 0; k < kIlp; ++k) {
+      const uint64_t b = lo + (uint64_t)(r + k) * w;
+      at[k] = 0;
+      len[k] = r + k != own && b < hi ? min(w, hi - (uint32_t)b) : 0u;
+    }
+    for (uint32_t step = w; step; step >>= 1) {
+#pragma unroll
+      for (uint32_t k = 0; k < kIlp; ++k) {
+        if (at[k] + step > len[k]) continue;
+        const float4 q = v[lo + (r + k) * w + at[k] + step - 1u];
+        if (r + k < own ? !rec_less(e, q) : rec_less(q, e)) at[k] += step;
+      }
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kIlp; ++k) rank += at[k];
+  }
+  return rank;
+}
+
+// Canonical order of the queued cells.  Phase 1 sorts each unit in shared
+// memory (a bitonic network over keys) into big_scratch;
+// then each merge pass joins up to kBigWays runs into one: a record's place
+// is its index in its own run plus its rank in the others.  After a cell's
+// last pass its run lies in big_buffer(passes), newborn marks kept, where
+// the pair search reads it, and in the next state without them.  False when
+// a grid barrier ran out (the same answer in every CTA that returns).
+template <bool kBinned>
+__device__ bool big_sort(const KParams& p, DevCtrl* c, uint32_t nbig, uint32_t units,
+                         unsigned long long* s_key) {
+  __shared__ BigCell s_big;
+  float4* nx = next_state(p, ld_u32(&c->cur));
+  const uint32_t passes = big_passes(ld_u32(&c->big_max));
+  for (uint32_t u = blockIdx.x; u < units; u += gridDim.x) {
+    __syncthreads();  // s_big and s_key of the last unit are no longer read
+    if (threadIdx.x == 0) s_big = big_unit(p, nbig, u);
+    __syncthreads();
+    const BigCell b = s_big;
+    if ((uint64_t)b.cs + b.n > p.capacity || b.first >= b.n) {
+      if (threadIdx.x == 0) atomicOr(&c->status, kStatBounds);
+      continue;  // uniform over the CTA
+    }
+    const uint32_t len = min(kBigChunk, b.n - b.first);
+    uint32_t size = 64;
+    while (size < len) size <<= 1;
+    const CellView cb = cell_records<kBinned>(p, b.cell, b.cs);
+    // Keys (x bits, index) through the network instead of whole records:
+    // half the shared-memory traffic and one comparison per exchange.
+    for (uint32_t i = threadIdx.x; i < size; i += blockDim.x)
+      s_key[i] = i < len ? (unsigned long long)__float_as_uint(cb[b.first + i].x) << 32 | i : ~0ull;
+    __syncthreads();
+    for (uint32_t k = 2; k <= size; k <<= 1) {
+      for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+        for (uint32_t t = threadIdx.x; t < size / 2; t += blockDim.x) {
+          const uint32_t i = ((t & ~(j - 1u)) << 1) | (t & (j - 1u)), ixj = i | j;
+          const unsigned long long q0 = s_key[i], q1 = s_key[ixj];
+          const bool swap = (q1 < q0) == ((i & k) == 0);
+          s_key[i] = swap ? q1 : q0;
+          s_key[ixj] = swap ? q0 : q1;
+        }
+        __syncthreads();
+      }
+    }
+    const bool done = b.n <= kBigChunk;
+    float4* tmp = big_buffer(p, b.cs, 0) + b.first;
+    for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) {
+      const unsigned long long key = s_key[i];
+      const float4 r = cb[b.first + (uint32_t)key];
+      // records with the same x bits are placed by all four words (by index
+      // when identical), counted over their stretch of equal keys
+      uint32_t at = i, lo = i, hi = i + 1u;
+      const uint32_t xb = (uint32_t)(key >> 32);
+      while (lo > 0 && (uint32_t)(s_key[lo - 1u] >> 32) == xb) --lo;
+      while (hi < len && (uint32_t)(s_key[hi] >> 32) == xb) ++hi;
+      if (hi - lo > 1u) {
+        at = lo;
+        for (uint32_t m = lo; m < hi; ++m) {
+          const float4 q = cb[b.first + (uint32_t)s_key[m]];
+          at += rec_less(q, r) || (m < i && rec_equal(q, r)) ? 1u : 0u;
+        }
+      }
+      tmp[at] = r;
+      if (done) nx[b.cs + b.first + at] = make_float4(r.x, r.y, r.z, __uint_as_float(rec_w(r) & ~kNewborn));
+    }
+  }
+  // few units: several CTAs share one unit's records
+  const uint32_t split = min(max(gridDim.x / units, 1u), kBigChunk / 256u), piece = (kBigChunk + split - 1u) / split;
+  uint32_t w = kBigChunk;
+  for (uint32_t pass = 0; pass < passes; ++pass, w *= kBigWays) {
+    if (!grid_barrier(c)) return false;
+    for (uint32_t job = blockIdx.x; job < units * split; job += gridDim.x) {
+      __syncthreads();
+      if (threadIdx.x == 0) s_big = big_unit(p, nbig, job / split);
+      __syncthreads();
+      const BigCell b = s_big;
+      if ((uint64_t)b.cs + b.n > p.capacity || b.n <= w) continue;
+      const float4* src = big_buffer(p, b.cs, pass);
+      float4* dst = big_buffer(p, b.cs, pass + 1u);
+      const uint64_t span = (uint64_t)w * kBigWays;
+      const bool last = span >= b.n;
+      const uint32_t begin = b.first + (job % split) * piece;
+      const uint32_t end = min(min(begin + piece, b.first + kBigChunk), b.n);
+      for (uint32_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
+        const float4 e = src[i];
+        const uint32_t lo = (uint32_t)(i / span * span), hi = (uint32_t)min((uint64_t)b.n, lo + span);
+        const uint32_t own = (i - lo) / w;
+        const uint32_t at = lo + (i - lo - own * w) + runs_rank(src, w, lo, hi, own, e);
+        dst[at] = e;
+        if (last) nx[b.cs + at] = make_float4(e.x, e.y, e.z, __uint_as_float(rec_w(e) & ~kNewborn));
+      }
+    }
+  }
+  return true;
+}
+// CTA-uniform status read (the large-cell kernel uses barriers).
 __device__ __forceinline__ bool stop_block(const DevCtrl* c) {
   __shared__ uint32_t s_stop;
   if (threadIdx.x == 0) s_stop = ld_u32(&c->status);
@@ -1536,200 +1702,279 @@ __device__ __forceinline__ bool stop_block(const DevCtrl* c) {
   return stop;
 }
 
-// Large cells, part 1 of 2 (k_pairs_big): the cells queued by
-// k_pairs_cells (more than kBigCell records, e.g. particles released at one
-// point), one CTA per cell, sorted in O(n log^2 n) rather than ranked in
-// O(n^2):
-//   1. chunks of 2048 records are sorted in shared memory (bitonic network,
-//      padded with all-ones records) into big_scratch;
-//   2. merge passes (each record finds its place in the partner run by
-//      binary search) double the sorted runs, alternating between
-//      big_scratch and the next state, until the cell is one canonical run;
-//   3. the run is left in both places: in the next state without newborn
-//      marks, in big_scratch (indexed by canonical slot) with them, where
-//      part 2 reads it.
+// What the lanes of a warp look for in a list of records: their own
+// seekers (lane on), the window on x that holds every partner of any of
+// them, and the species any of them reacts with.
+struct WarpSeekers {
+  Seeker k;
+  uint32_t ca;       // canonical slot of the lane's seeker
+  uint32_t partners; // bit s: some lane's species reacts with species s (all ones when S > 32)
+  float lo, hi;
+};
+
+__device__ __forceinline__ float warp_min(float v) {
+#pragma unroll
+  for (int d = 16; d; d >>= 1) v = fminf(v, __shfl_xor_sync(kFull, v, d));
+  return v;
+}
+
+// The warp's seekers (lanes `on`) against records [m0, m1) of the list v.
+// Each lane loads one record and drops it unless it lies in the warp's x
+// window and is of a species some lane reacts with; the few that remain
+// are passed around and tested by every lane, so records of species that
+// do not react cost a thirty-second of a test.  kRun: v is the canonical
+// run of a large cell (slots base + m), and only records past `after` (the
+// lane's own index, or -1) count; else an ordinary cell of nn records.
+template <bool kRun, class List>
+__device__ void warp_sweep(const KParams& p, DevCtrl* c, const WarpSeekers& s, bool on, const List v,
+                           uint32_t m0, uint32_t m1, uint32_t base, uint32_t nn, int64_t after) {
+  constexpr uint32_t kBatch = 4;  // loads in flight per lane (k_pairs_big 350 -> 282 us on the release below)
+  const uint32_t lane = lane_id();
+  const float4 none = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(kDead));
+  for (uint32_t m = m0; m < m1; m += 32u * kBatch) {
+    float4 q[kBatch];
+#pragma unroll
+    for (uint32_t u = 0; u < kBatch; ++u) q[u] = m1 - m > 32u * u + lane ? v[m + 32u * u + lane] : none;
+#pragma unroll
+    for (uint32_t u = 0; u < kBatch; ++u) {
+      const uint32_t wq = rec_w(q[u]), sp = wq & kSpeciesMask;
+      uint32_t ball = __ballot_sync(kFull, wq != kDead && !(wq & kNewborn) && q[u].x >= s.lo && q[u].x <= s.hi &&
+                                               (p.S > 32u || ((s.partners >> sp) & 1u)));
+      while (ball) {
+        const uint32_t src = (uint32_t)(__ffs(ball) - 1), at = m + 32u * u + src;
+        ball &= ball - 1u;
+        float4 r;
+        r.x = __shfl_sync(kFull, q[u].x, src);
+        r.y = __shfl_sync(kFull, q[u].y, src);
+        r.z = __shfl_sync(kFull, q[u].z, src);
+        r.w = __shfl_sync(kFull, q[u].w, src);
+        if (!on || (kRun && (int64_t)at <= after)) continue;
+        // |dy| bounds the distance as |dx| does; the pair test decides
+        if (fabsf(__fsub_rn(r.y, s.k.r.y)) > s.k.xlim) continue;
+        const int32_t b = pair_reaction(p, s.k, r);
+        if (b < 0) continue;
+        emit<false>(p, c, s.k, s.ca, base + (kRun ? at : canonical_rank(v, 0, nn, at, r)), b);
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// The records of [lo, hi) of the run v whose |x| lies in [t0, t1], as
+// [*a, *b); |x| rises over the range.  The whole warp searches both ends
+// together, 16 probes each a round.
+__device__ __forceinline__ void warp_range(const float4* v, uint32_t lo, uint32_t hi, float t0, float t1, uint32_t* a,
+                                           uint32_t* b) {
+  const uint32_t half = lane_id() >> 4, k = lane_id() & 15u;
+  uint32_t l = lo, h = hi;  // the lane's half: 0 looks for the first >= t0, 1 for the first > t1
+  while (__any_sync(kFull, l < h)) {
+    const uint32_t n = h - l, step = (n + 15u) >> 4;
+    bool below = false;
+    if (n) {
+      const float x = fabsf(v[l + min((k + 1u) * step, n) - 1u].x);  // last record of the lane's piece
+      below = half ? x <= t1 : x < t0;
+    }
+    const uint32_t ball = __ballot_sync(kFull, below) >> (half * 16u) & 0xFFFFu;
+    if (n) {
+      const uint32_t skip = min((uint32_t)__popc(ball) * step, n);  // pieces passed over whole
+      if (skip >= n) {
+        l = h;
+      } else {
+        h = min(l + skip + step, h) - 1u;  // the piece's last record is not below
+        l += skip;
+      }
+    }
+  }
+  *a = __shfl_sync(kFull, l, 0);
+  *b = __shfl_sync(kFull, l, 16);
+}
+
+// The sweep of a canonical run [0, n) of a large cell, restricted to the
+// warp's x window; segment `seg` of `nseg` takes its share of each of the
+// two ranges (x >= 0 ascending, then x < 0 by rising |x|).  from: no record
+// before it counts.
+__device__ void run_sweep(const KParams& p, DevCtrl* c, const WarpSeekers& s, bool on, const float4* v, uint32_t n,
+                          uint32_t base, uint32_t from, int64_t after, uint32_t seg, uint32_t nseg) {
+  // first record with the sign bit set
+  const float x0 = v[0].x, x1 = v[n - 1u].x;
+  uint32_t npos = n;
+  if (__float_as_uint(x0) & 0x80000000u) {
+    npos = 0;
+  } else if (__float_as_uint(x1) & 0x80000000u) {
+    uint32_t lo = 0, hi = n;
+    while (hi - lo > 0) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (__float_as_uint(v[mid].x) & 0x80000000u) hi = mid;
+      else lo = mid + 1u;
+    }
+    npos = lo;
+  }
+  for (int part = 0; part < 2; ++part) {
+    uint32_t a, b;
+    if (part == 0) {
+      if (npos == 0 || !(s.hi >= 0.0f)) continue;
+      warp_range(v, 0, npos, fmaxf(s.lo, 0.0f), s.hi, &a, &b);
+    } else {
+      if (npos == n || !(s.lo <= 0.0f)) continue;
+      warp_range(v, npos, n, fmaxf(-s.hi, 0.0f), -s.lo, &a, &b);
+    }
+    a = max(a, from);
+    if (a >= b) continue;
+    const uint32_t len = b - a;
+    const uint32_t m0 = a + (uint32_t)((uint64_t)len * seg / nseg), m1 = a + (uint32_t)((uint64_t)len * (seg + 1u) / nseg);
+    warp_sweep<true>(p, c, s, on, v, m0, m1, base, n, after);
+  }
+}
+
+// The warp's seekers: x window (widened past the rounding of x +- xlim;
+// xlim itself is 0.1% above the largest radius) and partner species.
+__device__ __forceinline__ void warp_seekers(const KParams& p, WarpSeekers& s, bool on, const uint32_t* s_partners) {
+  const float inf = __int_as_float(0x7f800000);
+  const float wx = on ? 1.001f * s.k.xlim + 1e-6f * fabsf(s.k.r.x) : 0.0f;
+  s.partners = __reduce_or_sync(kFull, on && p.S <= 32u ? s_partners[rec_w(s.k.r) & kSpeciesMask] : 0u);
+  s.lo = warp_min(on ? s.k.r.x - wx : inf);
+  s.hi = -warp_min(on ? -(s.k.r.x + wx) : inf);
+}
+
+// Neighbour cells that the largest binding radius of seeker k, in the cell
+// (cx, cy, cz), reaches: bit (dz * 3 + dy) * 3 + dx, offsets 0..2 for -1..+1.
+// An axis's distance counts only when it is within reach by itself (a record
+// past its face by rounding has a negative distance).
+__device__ __forceinline__ uint32_t big_mask(const KParams& p, const DevInstance& I, const Seeker& k, uint32_t cx,
+                                             uint32_t cy, uint32_t cz) {
+  const float inf = __int_as_float(0x7f800000);
+  const float cl0 = I.cell[0], cl1 = I.cell[1], cl2 = I.cell[2];
+  const float fx = __fsub_rn(__fmul_rn(__fsub_rn(k.r.x, I.lo[0]), I.inv[0]), (float)cx);
+  const float fy = __fsub_rn(__fmul_rn(__fsub_rn(k.r.y, I.lo[1]), I.inv[1]), (float)cy);
+  const float fz = __fsub_rn(__fmul_rn(__fsub_rn(k.r.z, I.lo[2]), I.inv[2]), (float)cz);
+  const float need = k.max_r + p.prune_margin * fminf(cl0, fminf(cl1, cl2)), need2 = need * need;
+  const float ex[3] = {cx > 0 ? fx * cl0 : inf, 0.0f, cx + 1u < I.dims[0] ? (1.0f - fx) * cl0 : inf};
+  const float ey[3] = {cy > 0 ? fy * cl1 : inf, 0.0f, cy + 1u < I.dims[1] ? (1.0f - fy) * cl1 : inf};
+  const float ez[3] = {cz > 0 ? fz * cl2 : inf, 0.0f, cz + 1u < I.dims[2] ? (1.0f - fz) * cl2 : inf};
+  uint32_t mask = 0;
+#pragma unroll
+  for (int t = 0; t < 27; ++t) {
+    const float dx = ex[t % 3], dy = ey[t / 3 % 3], dz = ez[t / 9];
+    if (t != 13 && dx <= need && dy <= need && dz <= need && dx * dx + dy * dy + dz * dz <= need2) mask |= 1u << t;
+  }
+  return mask;
+}
+
+// Pairs of the large cells, on the canonical runs big_sort left.  Each pair
+// that involves a large cell is tested once:
+//   * inside the cell, against the later records of the run;
+//   * with a large neighbour, from the lower-key cell of the two;
+//   * with an ordinary neighbour, here, in either direction (k_pairs_cells
+//     skips large forward neighbours).
+// Warps take 32 seekers at a time, consecutive in x, so that their windows
+// overlap.  Inside the cell these are 32 consecutive records.  For a
+// neighbour cell the CTA first lists the unit's records within reach of it
+// (a few per cent) and takes those 32 at a time: sweeping the neighbour for
+// every block of 32 records on behalf of the one or two lanes near it took
+// 160 of the kernel's 250 us.  With few units queued their work is spread
+// over more CTAs and a sweep over several warps.
 template <bool kBinned>
-__device__ void big_sort(const KParams& p, DevCtrl* c, uint32_t nbig, float4* s_rec) {
-  const uint32_t cur = ld_u32(&c->cur);
-  float4* nx = next_state(p, cur);
-  const float4 pad = make_float4(__uint_as_float(kFull), __uint_as_float(kFull), __uint_as_float(kFull),
-                                 __uint_as_float(kFull));
-  for (uint32_t bi = blockIdx.x; bi < nbig; bi += gridDim.x) {
-    const uint32_t cell = p.big[bi];
-    const uint32_t cs = p.cell_start[cell], n = p.cell_start[cell + 1] - cs;
-    if ((uint64_t)cs + n > p.capacity) {
-      if (threadIdx.x == 0) atomicOr(&c->status, kStatBounds);
-      continue;  // uniform over the CTA
-    }
-    const CellView cb = cell_records<kBinned>(p, cell, cs);
-    float4* out = nx + cs;
-    float4* tmp = p.big_scratch + cs;
-    for (uint32_t c0 = 0; c0 < n; c0 += kBigChunk) {
-      const uint32_t len = min(kBigChunk, n - c0);
-      for (uint32_t i = threadIdx.x; i < kBigChunk; i += blockDim.x) s_rec[i] = i < len ? cb[c0 + i] : pad;
-      __syncthreads();
-      for (uint32_t k = 2; k <= kBigChunk; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-          for (uint32_t i = threadIdx.x; i < kBigChunk; i += blockDim.x) {
-            const uint32_t ixj = i ^ j;
-            if (ixj > i) {
-              const float4 a = s_rec[i], b = s_rec[ixj];
-              const bool up = (i & k) == 0;
-              if (rec_less(b, a) == up) {
-                s_rec[i] = b;
-                s_rec[ixj] = a;
-              }
-            }
-          }
-          __syncthreads();
-        }
-      }
-      for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) tmp[c0 + i] = s_rec[i];
-      __syncthreads();
-    }
-    float4* src = tmp;
-    float4* dst = out;
-    for (uint32_t w = kBigChunk; w < n; w <<= 1) {
-      for (uint32_t idx = threadIdx.x; idx < n; idx += blockDim.x) {
-        const uint32_t lo = idx / (2 * w) * (2 * w);
-        const uint32_t mid = min(lo + w, n), hi = min(lo + 2 * w, n);
-        const float4 e = src[idx];
-        const uint32_t pos = idx < mid ? (idx - lo) + run_rank<false>(src + mid, hi - mid, e)
-                                       : (idx - mid) + run_rank<true>(src + lo, mid - lo, e);
-        dst[lo + pos] = e;
-      }
-      __syncthreads();
-      float4* t = src;
-      src = dst;
-      dst = t;
-    }
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-      const float4 r = src[i];
-      tmp[i] = r;
-      out[i] = make_float4(r.x, r.y, r.z, __uint_as_float(rec_w(r) & ~kNewborn));
+__device__ void big_pairs(const KParams& p, DevCtrl* c, uint32_t nbig, uint32_t units) {
+  constexpr uint32_t kWarps = 8, kPer = kBigChunk / 256u;  // CTAs of 256 threads; records of a unit per thread
+  __shared__ BigCell s_big;
+  __shared__ uint32_t s_partners[32], s_union, s_count[kPer * kWarps + 1];
+  __shared__ uint16_t s_list[kBigChunk];
+  // species a species reacts with, as bits
+  if (p.S <= 32u && threadIdx.x < p.S) {
+    uint32_t m = 0;
+    for (uint32_t t = 0; t < p.S; ++t) m |= (p.bim_table[threadIdx.x * p.S + t] >= 0 ? 1u : 0u) << t;
+    s_partners[threadIdx.x] = m;
+  }
+  const uint32_t parts = min(max(2u * gridDim.x / units, 1u), kBigParts);
+  const uint32_t nseg = parts > 1u ? kBigSegments : 1u;
+  const uint32_t own = (parts + 1u) / 2u, turns = min((parts + 1u) / 2u, 13u);  // CTAs on the own cell, on neighbours
+  const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
+  for (uint32_t job = blockIdx.x; job < units * (own + turns); job += gridDim.x) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_big = big_unit(p, nbig, job / (own + turns));
+      s_union = 0;
     }
     __syncthreads();
-  }
-}
-
-// Index of the first record of the sorted run [0, n) whose x has its sign
-// bit set: canonical order sorts x >= 0 ascending, then negative x by |x|.
-__device__ __forceinline__ uint32_t run_negative_start(const float4* run, uint32_t n) {
-  uint32_t lo = 0, hi = n;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (__float_as_uint(run[mid].x) & 0x80000000u) hi = mid;
-    else lo = mid + 1;
-  }
-  return lo;
-}
-
-// First record of [lo, hi) (sorted by |x| within one sign) with |x| >= v.
-__device__ __forceinline__ uint32_t run_abs_lower(const float4* run, uint32_t lo, uint32_t hi, float v) {
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (fabsf(run[mid].x) < v) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// Pairs of seeker k (canonical slot ca) with the records of a sorted run
-// (canonical slots base + m) whose |x - k.x| is within k.xlim, skipping
-// m <= skip_to (in-cell: only later records; else pass -1).
-template <bool kSingle>
-__device__ void sweep_sorted(const KParams& p, DevCtrl* c, const Seeker& k, uint32_t ca, const float4* run,
-                             uint32_t n, uint32_t base, int64_t skip_to) {
-  const uint32_t npos = run_negative_start(run, n);
-  // bounds widened well past any rounding of x0 +- xlim; the pair test decides
-  const float x0 = k.r.x, w = 2.0f * k.xlim + 1e-6f * fabsf(x0);
-  const float lo = x0 - w, hi = x0 + w;
-  if (hi >= 0.0f) {  // x >= 0 part, ascending
-    for (uint32_t m = run_abs_lower(run, 0, npos, fmaxf(lo, 0.0f)); m < npos; ++m) {
-      const float4 q = run[m];
-      if (q.x > hi) break;
-      if ((int64_t)m <= skip_to) continue;
-      const int32_t b = pair_reaction(p, k, q);
-      if (b >= 0) emit<kSingle>(p, c, k, ca, base + m, b);
-    }
-  }
-  if (lo <= 0.0f) {  // x < 0 part, ascending |x|
-    for (uint32_t m = run_abs_lower(run, npos, n, fmaxf(-hi, 0.0f)); m < n; ++m) {
-      const float4 q = run[m];
-      if (fabsf(q.x) > -lo) break;
-      if ((int64_t)m <= skip_to) continue;
-      const int32_t b = pair_reaction(p, k, q);
-      if (b >= 0) emit<kSingle>(p, c, k, ca, base + m, b);
-    }
-  }
-}
-
-// Large cells, part 2 of 2 (k_pairs_big), one CTA per queued cell, on the
-// canonical runs left by part 1.  Each pair involving a large cell is
-// tested once:
-//   * inside the cell, by x sweeps over the run;
-//   * with a large neighbour, from the lower-key cell of the two, by x
-//     sweeps over the neighbour's run (binary search to |dx| <= radius);
-//   * with an ordinary neighbour, here, in either direction, by a loop
-//     over its records (k_pairs_cells skips large forward neighbours).
-template <bool kBinned>
-__device__ void big_pairs(const KParams& p, DevCtrl* c, uint32_t nbig) {
-  for (uint32_t bi = blockIdx.x; bi < nbig; bi += gridDim.x) {
-    const uint32_t cell = p.big[bi];
-    const uint32_t cs = p.cell_start[cell], n = p.cell_start[cell + 1] - cs;
-    if ((uint64_t)cs + n > p.capacity) continue;
-    const float4* run = p.big_scratch + cs;
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-      Seeker k;
-      if (!seeker_init<false>(p, run[i], k)) continue;
-      const uint32_t ca = cs + i;
-      sweep_sorted<false>(p, c, k, ca, run, n, cs, (int64_t)i);
-      const DevInstance& I = p.inst[k.inst];
-      const float cl0 = I.cell[0], cl1 = I.cell[1], cl2 = I.cell[2];
-      const uint32_t d0 = I.dims[0], d1 = I.dims[1], d2 = I.dims[2];
-      const float gx = __fmul_rn(__fsub_rn(k.r.x, I.lo[0]), I.inv[0]);
-      const float gy = __fmul_rn(__fsub_rn(k.r.y, I.lo[1]), I.inv[1]);
-      const float gz = __fmul_rn(__fsub_rn(k.r.z, I.lo[2]), I.inv[2]);
-      const int cx = min(max((int)floorf(gx), 0), (int)d0 - 1);
-      const int cy = min(max((int)floorf(gy), 0), (int)d1 - 1);
-      const int cz = min(max((int)floorf(gz), 0), (int)d2 - 1);
-      const float margin = p.prune_margin * fminf(cl0, fminf(cl1, cl2));
-      const float need = k.max_r + margin, need2 = need * need;
-      const float fx = __fsub_rn(gx, (float)cx), fy = __fsub_rn(gy, (float)cy), fz = __fsub_rn(gz, (float)cz);
-      const float dlo[3] = {fx * cl0, fy * cl1, fz * cl2};
-      const float dhi[3] = {(1.0f - fx) * cl0, (1.0f - fy) * cl1, (1.0f - fz) * cl2};
-      const int c3[3] = {cx, cy, cz};
-      const int dm[3] = {(int)d0, (int)d1, (int)d2};
-      int lo3[3], hi3[3];
-      for (int a = 0; a < 3; ++a) {
-        lo3[a] = (c3[a] > 0 && dlo[a] <= need) ? -1 : 0;
-        hi3[a] = (c3[a] + 1 < dm[a] && dhi[a] <= need) ? 1 : 0;
+    const BigCell bc = s_big;
+    if ((uint64_t)bc.cs + bc.n > p.capacity || bc.first >= bc.n) continue;
+    const float4* run = big_buffer(p, bc.cs, big_passes(bc.n));
+    const uint32_t len = min(kBigChunk, bc.n - bc.first), part = job % (own + turns);
+    WarpSeekers s;
+    if (part < own) {
+      for (uint32_t item = part * kWarps + warp; item < (len + 31u) / 32u * nseg; item += own * kWarps) {
+        const uint32_t i0 = bc.first + item / nseg * 32u, i = i0 + lane;
+        s.ca = bc.cs + i;
+        const bool on = i < bc.n && seeker_init<false>(p, run[i], s.k);
+        if (!__any_sync(kFull, on)) continue;
+        warp_seekers(p, s, on, s_partners);
+        run_sweep(p, c, s, on, run, bc.n, bc.cs, i0 + 1u, (int64_t)i, item % nseg, nseg);
       }
-      for (int dz = lo3[2]; dz <= hi3[2]; ++dz) {
-        const float ddz = dz < 0 ? dlo[2] : (dz > 0 ? dhi[2] : 0.0f);
-        for (int dy = lo3[1]; dy <= hi3[1]; ++dy) {
-          const float ddy = dy < 0 ? dlo[1] : (dy > 0 ? dhi[1] : 0.0f);
-          for (int dx = lo3[0]; dx <= hi3[0]; ++dx) {
-            if (dx == 0 && dy == 0 && dz == 0) continue;
-            const float ddx = dx < 0 ? dlo[0] : (dx > 0 ? dhi[0] : 0.0f);
-            if (ddx * ddx + ddy * ddy + ddz * ddz > need2) continue;
-            const bool forward = dz > 0 || (dz == 0 && (dy > 0 || (dy == 0 && dx > 0)));
-            const uint32_t nkey =
-                I.cell_base + ((uint32_t)(cz + dz) * d1 + (uint32_t)(cy + dy)) * d0 + (uint32_t)(cx + dx);
-            const uint32_t ns = __ldg(&p.cell_start[nkey]), nn = __ldg(&p.cell_start[nkey + 1]) - ns;
-            if (nn > kBigCell) {
-              if (forward) sweep_sorted<false>(p, c, k, ca, p.big_scratch + ns, nn, ns, -1);
-              continue;  // a large lower-key neighbour finds this pair itself
-            }
-            const CellView nb = cell_records<kBinned>(p, nkey, ns);
-            for (uint32_t m = 0; m < nn; ++m) {
-              const float4 q = nb.ldg(m);
-              const int32_t b = pair_reaction(p, k, q);
-              if (b >= 0) emit<false>(p, c, k, ca, ns + canonical_rank(nb, 0, nn, m, q), b);
-            }
-          }
+      continue;
+    }
+    // the records near each neighbour; every record of a cell has its instance
+    const DevInstance& I = p.inst[rec_w(run[0]) >> 16];
+    const uint32_t d0 = I.dims[0], d1 = I.dims[1], local = bc.cell - I.cell_base;
+    const uint32_t cx = local % d0, cy = local / d0 % d1, cz = local / d0 / d1;
+    uint32_t mask[kPer], any = 0;
+#pragma unroll
+    for (uint32_t e = 0; e < kPer; ++e) {
+      const uint32_t i = e * 256u + threadIdx.x;
+      mask[e] = i < len && seeker_init<false>(p, run[bc.first + i], s.k) ? big_mask(p, I, s.k, cx, cy, cz) : 0u;
+      any |= mask[e];
+    }
+    any = __reduce_or_sync(kFull, any);
+    if (lane == 0 && any) atomicOr(&s_union, any);
+    __syncthreads();
+    uint32_t todo = s_union;
+    for (uint32_t turn = 0; todo; ++turn) {  // the same in every thread of the CTA
+      const uint32_t t = (uint32_t)(__ffs(todo) - 1);
+      todo &= todo - 1u;
+      if (turn % turns != part - own) continue;
+      const uint32_t nkey =
+          bc.cell + (uint32_t)(((int)(t / 9u) - 1) * (int)d1 + ((int)(t / 3u % 3u) - 1)) * d0 + t % 3u - 1u;
+      const uint32_t ns = __ldg(&p.cell_start[nkey]), nn = __ldg(&p.cell_start[nkey + 1]) - ns;
+      const bool large = nn > kBigCell;
+      if (nn == 0 || (large && t < 13u)) continue;  // a large lower-key neighbour finds the pair itself
+#pragma unroll
+      for (uint32_t e = 0; e < kPer; ++e) {
+        const uint32_t ball = __ballot_sync(kFull, (mask[e] >> t) & 1u);
+        if (lane == 0) s_count[e * kWarps + warp] = __popc(ball);
+      }
+      __syncthreads();
+      if (warp == 0) {  // exclusive scan of the 64 counts
+        const uint32_t a = s_count[2u * lane], b = s_count[2u * lane + 1u];
+        uint32_t incl = a + b;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const uint32_t v = __shfl_up_sync(kFull, incl, d);
+          if (lane >= (uint32_t)d) incl += v;
         }
+        s_count[2u * lane] = incl - a - b;
+        s_count[2u * lane + 1u] = incl - b;
+        if (lane == 31) s_count[kPer * kWarps] = incl;
       }
+      __syncthreads();
+#pragma unroll
+      for (uint32_t e = 0; e < kPer; ++e) {
+        const bool hit = (mask[e] >> t) & 1u;
+        const uint32_t ball = __ballot_sync(kFull, hit);
+        if (hit) s_list[s_count[e * kWarps + warp] + __popc(ball & ((1u << lane) - 1u))] = (uint16_t)(e * 256u + threadIdx.x);
+      }
+      __syncthreads();
+      const uint32_t m = s_count[kPer * kWarps], blocks = (m + 31u) / 32u;
+      const uint32_t cut = large ? max(kWarps / blocks, 1u) : 1u;
+      for (uint32_t item = warp; item < blocks * cut; item += kWarps) {
+        const uint32_t j = item / cut * 32u + lane;
+        const uint32_t i = bc.first + (j < m ? s_list[j] : 0u);
+        s.ca = bc.cs + i;
+        const bool on = j < m && seeker_init<false>(p, run[i], s.k);
+        if (!__any_sync(kFull, on)) continue;
+        warp_seekers(p, s, on, s_partners);
+        if (large) run_sweep(p, c, s, on, big_buffer(p, ns, big_passes(nn)), nn, ns, 0u, -1, item % cut, cut);
+        else warp_sweep<false>(p, c, s, on, cell_records<kBinned>(p, nkey, ns), 0u, nn, ns, nn, -1);
+      }
+      __syncthreads();  // s_count and s_list are no longer read
     }
   }
 }
@@ -1744,19 +1989,20 @@ __device__ void big_pairs(const KParams& p, DevCtrl* c, uint32_t nbig) {
 // raises kStatScratch; the host allocates it and replays the step.
 template <bool kHasBim, bool kBinned>
 __global__ void __launch_bounds__(256) k_pairs_big(KParams p) {
-  __shared__ float4 s_rec[kBigChunk];
+  __shared__ unsigned long long s_key[kBigChunk];
   DevCtrl* c = p.ctrl;
   if (stop_block(c)) return;
-  const uint32_t nbig = min(ld_u32(&c->n_big), p.big_cap);
+  const unsigned long long queued = __ldcg(&c->big_queue);
+  const uint32_t nbig = min((uint32_t)queued, p.big_cap), units = (uint32_t)(queued >> 32);
   if (nbig == 0) return;
-  if (p.big_scratch_cap < p.capacity) {
+  if (p.big_scratch_cap < 2ull * p.capacity) {
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&c->status, kStatScratch);
     return;
   }
-  big_sort<kBinned>(p, c, nbig, s_rec);
+  if (!big_sort<kBinned>(p, c, nbig, units, s_key)) return;
   if (!kHasBim) return;
   if (!grid_barrier(c)) return;
-  big_pairs<kBinned>(p, c, nbig);
+  big_pairs<kBinned>(p, c, nbig, units);
 }
 
 // Move the events of the committed step into the cumulative counters.
@@ -2006,7 +2252,8 @@ __global__ void __launch_bounds__(1024) k_match(KParams p) {
   if (threadIdx.x == 0) {
     c->n_pairs_last = K;
     c->n_pairs = 0;
-    c->n_big = 0;
+    c->big_queue = 0;
+    c->big_max = 0;
     c->n_surf = 0;
     c->surf_ticket = 0;
     c->deaths_last = s_deaths;

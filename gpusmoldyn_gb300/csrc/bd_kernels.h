@@ -43,9 +43,10 @@ struct KParams {
   uint32_t n_cells, n_tiles;
   uint32_t capacity, pair_cap;
   uint32_t bin_cap;           // records per cell bin (binned sort)
-  uint32_t* big;              // [big_cap] cells queued for k_pairs_big
-  float4* big_scratch;        // [big_scratch_cap] merge-sort buffer of k_pairs_big
-  uint32_t big_cap, big_scratch_cap;
+  uint2* big;                 // [big_cap] (cell, first unit) queued for k_pairs_big
+  float4* big_scratch;        // [big_scratch_cap] sort buffers of k_pairs_big, two of [capacity]
+  uint32_t big_cap;
+  uint64_t big_scratch_cap;
   float prune_margin;         // fraction of a cell edge added to pruning distances
   // surfaces (n_panels = 0: none)
   const DevPanel* panels;     // [n_panels]

@@ -107,9 +107,12 @@ struct DevCtrl {
   uint32_t status;         // StatusBits, 0 = healthy
   uint32_t steps_done;     // completed steps since the last host reset
   uint64_t step;           // global step counter
+  // large cells queued for k_pairs_big: units (high word) and cells (low
+  // word), and the most records of one
+  unsigned long long big_queue;
+  uint32_t big_max;
   uint32_t deaths_last;    // bimolecular deaths of the last step
   uint32_t bin_need;       // largest cell occupancy seen by a bin that overflowed
-  uint32_t n_big;          // cells queued for the large-cell pair kernel
   uint32_t n_surf;         // records whose move meets a panel box (binned path with surfaces)
   uint32_t surf_ticket;    // queued records taken by k_bin_surface in the step in flight
   // the grid barrier (cell scan; k_match over the whole grid when a step
