@@ -32,6 +32,12 @@ using namespace bd;
 namespace {
 
 constexpr int kGraphBatch = 16;
+// Cells up to which a binned step runs in k_resident.  A c2 step takes, there
+// and as a chain of kernels (us): 1,000 particles 10.4 / 23.6, 100,000 23.5 /
+// 32.2, 1M (333,333 cells) 54.2 / 56.0, 1.2M 59.7 / 60.3, 2M 90.9 / 83.9.
+constexpr uint32_t kResidentCells = 400000;
+// Mean zeroth-order births per step up to which it does.
+constexpr double kResidentBirths = 4096.0;
 // Largest bin array the automatic sort mode accepts.
 constexpr uint64_t kBinBudgetBytes = 32ull << 30;
 
@@ -136,7 +142,7 @@ struct bd_system {
   DevBuf<DevPair> pairs;
 
   std::vector<DevInstance> hinst;
-  uint32_t n_cells = 0, n_tiles = 0;
+  uint32_t n_cells = 0, n_tiles = 0, count_stride = 0;
   uint64_t capacity = 0;
   uint32_t pair_cap = 0;
   bool binned = false;             // Path::kBinned (else the compact counting sort)
@@ -167,7 +173,18 @@ struct bd_system {
   bool diffuse_only() const {
     return U == 0 && B == 0 && idesc.size() == 1 && !zero_two_products && !server && panels.empty();
   }
-  Path path() const { return diffuse_only() ? Path::kDiffuseOnly : (binned ? Path::kBinned : Path::kSorted); }
+  // The binned step of a small system runs in k_resident: no panels (their
+  // walk needs more registers than the resident phases have), few births a
+  // step (one CTA makes them), and small enough that launches and latency
+  // outweigh the work.
+  double births = 0.0;  // mean zeroth-order births per step
+  bool resident() const {
+    return binned && panels.empty() && n_cells <= kResidentCells && births <= kResidentBirths && shape.grid_resident > 0;
+  }
+  Path path() const {
+    return diffuse_only() ? Path::kDiffuseOnly
+                          : (binned ? (resident() ? Path::kResident : Path::kBinned) : Path::kSorted);
+  }
   int n_inst() const { return (int)idesc.size(); }
 };
 
@@ -212,6 +229,7 @@ KParams make_params(bd_system* h) {
   p.inst_slot_base = h->inst_slot_base.p;
   p.zero_off = h->zero_off.p;
   p.cell_count = h->cell_count.p;
+  p.count_stride = h->count_stride;
   p.cell_start = h->cell_start.p;
   p.tile_sums = h->tile_sums.p;
   p.scan_withhold = h->scan_withhold ? 1u : 0u;
@@ -260,6 +278,7 @@ bd_status build_graphs(bd_system* h) {
       memcmp(&h->shape, &h->graph_shape, sizeof h->shape) == 0)
     return BD_OK;
   destroy_graphs(h);
+  if (path == Path::kResident) return BD_OK;  // launched directly
   const bool has_zero = h->Z > 0, has_uni = h->U > 0, has_bim = h->B > 0;
   for (int g = 0; g < 2; g++) {
     const int nsteps = g == 0 ? 1 : kGraphBatch;
@@ -406,6 +425,7 @@ bd_status create_common(const bd_config* cfg, const bd_instance_desc* inst, int 
   h->shape.grid_match = h->host_only ? 1 : match_grid(h->n_sm);
   h->shape.grid_scan = h->host_only ? 1 : scan_grid(h->n_sm);
   h->shape.grid_big = h->host_only ? 1 : big_grid(h->n_sm);
+  h->shape.grid_resident = h->host_only ? 0 : resident_grid(h->n_sm);
   memset(h->hctrl, 0, sizeof(DevCtrl));
   cudaMemset(h->ctrl.p, 0, sizeof(DevCtrl));
   *out = h;
@@ -527,17 +547,23 @@ bd_status layout_cells(bd_system* h) {
   if (base > 0xFFFFFFF0ull) return BD_ERR_CAPACITY;
   h->n_cells = (uint32_t)base;
   h->n_tiles = (uint32_t)((base + kScanTile - 1) / kScanTile);
+  h->births = 0.0;
+  for (int k = 0; k < I; k++)
+    if (!h->server || h->slot_used[k])
+      for (int z : h->zero_list) h->births += h->derived[k].rx[z].prob;
   if (h->host_only) return BD_OK;
   // grow-only: a serving handle lays its cells out again at every admission,
   // and cudaFree would wait for the whole device
   auto ensure = [](auto& buf, size_t count) { return buf.p && buf.n >= count ? cudaSuccess : buf.alloc(count); };
   BD_CUDA(ensure(h->dinst, (size_t)I));
   BD_CUDA(cudaMemcpyAsync(h->dinst.p, h->hinst.data(), I * sizeof(DevInstance), cudaMemcpyHostToDevice, h->stream));
-  BD_CUDA(ensure(h->cell_count, (size_t)h->n_cells));
-  BD_CUDA(cudaMemsetAsync(h->cell_count.p, 0, (size_t)h->n_cells * sizeof(uint32_t), h->stream));
+  // two count arrays (k_resident), 16-byte aligned
+  h->count_stride = (h->n_cells + kCellPad + 3u) & ~3u;
+  BD_CUDA(ensure(h->cell_count, 2 * (size_t)h->count_stride));
+  BD_CUDA(cudaMemsetAsync(h->cell_count.p, 0, 2 * (size_t)h->count_stride * sizeof(uint32_t), h->stream));
   BD_CUDA(ensure(h->cell_start, (size_t)h->n_cells + 1));
   BD_CUDA(cudaMemsetAsync(h->cell_start.p, 0, ((size_t)h->n_cells + 1) * sizeof(uint32_t), h->stream));
-  BD_CUDA(ensure(h->tile_sums, (size_t)std::max<uint32_t>(h->n_tiles, 1)));
+  BD_CUDA(ensure(h->tile_sums, (size_t)std::max<uint32_t>(h->n_tiles, (uint32_t)std::max(h->shape.grid_resident, 1))));
   BD_CUDA(cudaStreamSynchronize(h->stream));
   if (!h->panels.empty()) {
     const bd_status st = upload_cell_masks(h);
@@ -1194,11 +1220,20 @@ BD_API bd_status bd_step(bd_handle h, int nsteps) {
   if (h->host_only) return BD_ERR_NO_DEVICE;
   if (!h->have_particles) return BD_ERR_NOT_FINALIZED;
   BD_CUDA(cudaSetDevice(h->device));
+  int left = nsteps;
+  if (h->path() == Path::kResident) {
+    const KParams p = make_params(h);
+    for (; left > 0; left -= (int)kResidentSteps)
+      enqueue_resident(p, h->cfg.normal_mode == BD_NORMALS_TABLE, h->B > 0,
+                       (uint32_t)std::min(left, (int)kResidentSteps), h->hctrl->n_slots, h->shape, h->stream);
+    BD_CUDA(cudaGetLastError());
+    h->target_step += (uint64_t)nsteps;
+    return BD_OK;
+  }
   if (!h->graph1) {
     const bd_status st = build_graphs(h);
     if (st) return st;
   }
-  int left = nsteps;
   while (left >= kGraphBatch) {
     BD_CUDA(cudaGraphLaunch(h->graphN, h->stream));
     left -= kGraphBatch;
@@ -1223,10 +1258,6 @@ BD_API bd_status bd_measure_msd(bd_handle h, int inst, int nsteps, double* msd, 
   BD_CUDA(cudaSetDevice(h->device));
   bd_status st = bd_synchronize(h);
   if (st && st != BD_ERR_EMPTY) return st;
-  if (!h->graph1) {
-    st = build_graphs(h);
-    if (st) return st;
-  }
   const size_t m = (size_t)h->n_inst() * h->S;
   DevBuf<double> sum;
   DevBuf<unsigned long long> cnt;
@@ -1242,12 +1273,7 @@ BD_API bd_status bd_measure_msd(bd_handle h, int inst, int nsteps, double* msd, 
     // replay repeats the same moves unmeasured
     enqueue_msd(make_params(h), table, sum.p, cnt.p, h->stream);
     BD_CUDA(cudaGetLastError());
-    if (!h->graph1) {
-      st = build_graphs(h);
-      if (st) return st;
-    }
-    BD_CUDA(cudaGraphLaunch(h->graph1, h->stream));
-    h->target_step += 1;
+    if ((st = bd_step(h, 1))) return st;
     st = bd_synchronize(h);
     if (st && st != BD_ERR_EMPTY) return st;
   }
@@ -1342,7 +1368,7 @@ BD_API bd_status bd_synchronize(bd_handle h) {
         st = grow_pairs(h, (uint32_t)cap);
         if (st) return st;
       }
-      BD_CUDA(cudaMemsetAsync(h->cell_count.p, 0, (size_t)h->n_cells * sizeof(uint32_t), h->stream));
+      BD_CUDA(cudaMemsetAsync(h->cell_count.p, 0, 2 * (size_t)h->count_stride * sizeof(uint32_t), h->stream));
       BD_CUDA(cudaMemsetAsync(h->pending.p, 0, h->pending.n * sizeof(unsigned long long), h->stream));
       c.status = 0;
       c.n_pairs = 0;
@@ -1352,6 +1378,8 @@ BD_API bd_status bd_synchronize(bd_handle h) {
       c.surf_ticket = 0;
       c.n_virtual = 0;
       c.bar_count = 0;
+      c.res_word = 0;
+      c.res_left = 0;
       st = push_ctrl(h);
       if (st) return st;
       st = build_graphs(h);
@@ -1902,8 +1930,13 @@ BD_API bd_status bd_profile_steps(bd_handle h, int nsteps, float* stage_ms, int 
     BD_CUDA(cudaEventRecord(e0, h->stream));
     ev.push_back(e0);
     ProfileCtx ctx{h->stream, &ev, &h->stage_names, k == 0};
-    const int nk = enqueue_step(p, path, table, h->Z > 0, h->U > 0, h->B > 0, h->shape, h->stream, profile_hook,
-                                &ctx);
+    int nk = 1;
+    if (path == Path::kResident) {
+      enqueue_resident(p, table, h->B > 0, 1, h->hctrl->n_slots, h->shape, h->stream);
+      profile_hook(&ctx, "k_resident");
+    } else {
+      nk = enqueue_step(p, path, table, h->Z > 0, h->U > 0, h->B > 0, h->shape, h->stream, profile_hook, &ctx);
+    }
     BD_CUDA(cudaGetLastError());
     BD_CUDA(cudaEventSynchronize(ev.back()));
     if (acc.empty()) acc.assign(nk, 0.0f);
@@ -1930,6 +1963,7 @@ BD_API const char* bd_stage_name(bd_handle h, int k) {
 BD_API bd_status bd_get_kernels_per_step(bd_handle h, int* n) {
   if (!h || !n) return BD_ERR_INVALID_ARGUMENT;
   if (h->diffuse_only()) *n = (h->Z > 0 ? 2 : 0) + 2;
+  else if (h->path() == Path::kResident) *n = 1;
   // binned: k_bin, k_scan, k_pairs_cells, k_pairs_big, k_match (+ k_bin_surface
   // with panels); compact: k_count, k_scan, k_scatter, k_pairs_cells,
   // k_pairs_big, k_match; k_zeroth first with zeroth-order reactions

@@ -30,6 +30,7 @@ struct KParams {
   uint32_t* zero_off;         // [I*Z + 1] prefix of zeroth-order births
   DevZero zero0[4];           // instance 0's zeroth-order entries when Z <= 4 (k_zeroth's one-instance path)
   uint32_t* cell_count;       // [n_cells] particles per cell (returns to 0 each step)
+  uint32_t count_stride;      // words to the second count array (k_resident alternates between them)
   uint32_t* cell_start;       // [n_cells + 1] exclusive prefix of cell_count
   uint32_t* tile_sums;        // [n_tiles] the cell scan's per-CTA sums
   uint32_t scan_withhold;     // test switch: CTA 0 of the cell scan never reaches its grid barrier
@@ -64,7 +65,9 @@ struct KParams {
 // k_scatter) before the pair kernel.  kBinned: each record goes straight
 // into a fixed-size bin of its cell (k_bin), the scans give the compact
 // output ranges and the pair kernel reads the bins.  Same results.
-enum class Path { kDiffuseOnly, kSorted, kBinned };
+// kResident: the binned step of a small system, many steps per launch
+// (bd_resident.cu).
+enum class Path { kDiffuseOnly, kSorted, kBinned, kResident };
 
 struct LaunchShape {
   int grid_stream;            // blocks of the grid-stride particle kernels
@@ -74,6 +77,7 @@ struct LaunchShape {
   int grid_match;             // CTAs of the cooperative matcher (1 = one CTA, plain launch)
   int grid_scan;              // most CTAs of the cooperative cell scan (all resident)
   int grid_big;               // CTAs of the large-cell kernel (all resident)
+  int grid_resident;          // most CTAs of k_resident (all resident)
 };
 
 // CTAs of 1024 threads that the matcher can keep resident on n_sm SMs (the
@@ -83,6 +87,12 @@ int match_grid(int n_sm);
 int scan_grid(int n_sm);
 // CTAs of the large-cell kernel: at most 304, all resident on n_sm SMs.
 int big_grid(int n_sm);
+// CTAs of 1024 threads, at most one per SM, that k_resident can keep resident on n_sm SMs.
+int resident_grid(int n_sm);
+// Most steps of one launch of k_resident: long enough to hide the launch,
+// short enough to let other streams in.  Most reactions of its one-instance
+// variant.
+constexpr uint32_t kResidentSteps = 64, kResidentReactions = 128;
 
 // Called after each kernel of a step is enqueued (stage name); lets the
 // profiler record an event between kernels.  nullptr = no callback.
@@ -92,6 +102,11 @@ typedef void (*StageHook)(void* ctx, const char* stage);
 // Returns the number of kernels enqueued.
 int enqueue_step(const KParams& p, Path path, bool table, bool has_zero, bool has_uni, bool has_bim,
                  const LaunchShape& shape, cudaStream_t stream, StageHook hook = nullptr, void* ctx = nullptr);
+
+// nsteps steps of a small binned system of about n_slots records, in one
+// launch of k_resident.
+void enqueue_resident(const KParams& p, bool table, bool has_bim, uint32_t nsteps, uint64_t n_slots,
+                      const LaunchShape& shape, cudaStream_t stream);
 
 // Count live records per instance (counts[I] must be zeroed).
 void enqueue_instance_counts(const KParams& p, unsigned long long* counts, cudaStream_t stream);
@@ -103,6 +118,10 @@ void enqueue_msd(const KParams& p, bool table, double* sum, unsigned long long* 
 
 // Tile size of the cell scan.
 constexpr uint32_t kScanTile = 8192;
+
+// Entries past the cells in the count arrays (always 0), so that counts can be
+// read four at a time.
+constexpr uint32_t kCellPad = 8;
 
 // Places of a cell bin stored together (64 bytes); the bin capacity is a
 // multiple of it.

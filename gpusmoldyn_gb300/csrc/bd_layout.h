@@ -121,6 +121,9 @@ struct DevCtrl {
   uint32_t bar_count, bar_gen;
   uint32_t match_next[2];
   uint32_t match_deaths;
+  // k_resident: the arrival word of its barriers and the CTAs that have left
+  unsigned long long res_word;
+  uint32_t res_left;
 };
 
 enum StatusBits : uint32_t {
