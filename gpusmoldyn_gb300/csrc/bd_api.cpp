@@ -278,7 +278,7 @@ bd_status build_graphs(bd_system* h) {
       memcmp(&h->shape, &h->graph_shape, sizeof h->shape) == 0)
     return BD_OK;
   destroy_graphs(h);
-  if (path == Path::kResident) return BD_OK;  // launched directly
+  if (path == Path::kResident || (path == Path::kDiffuseOnly && h->Z == 0)) return BD_OK;  // launched directly
   const bool has_zero = h->Z > 0, has_uni = h->U > 0, has_bim = h->B > 0;
   for (int g = 0; g < 2; g++) {
     const int nsteps = g == 0 ? 1 : kGraphBatch;
@@ -1230,6 +1230,16 @@ BD_API bd_status bd_step(bd_handle h, int nsteps) {
     h->target_step += (uint64_t)nsteps;
     return BD_OK;
   }
+  if (h->path() == Path::kDiffuseOnly && h->Z == 0) {
+    // no reaction changes the slot count: the host's copy is right
+    const KParams p = make_params(h);
+    for (; left > 0; left -= (int)kDiffuseSteps)
+      enqueue_diffuse(p, h->cfg.normal_mode == BD_NORMALS_TABLE, (uint32_t)std::min(left, (int)kDiffuseSteps),
+                      h->hctrl->n_slots, h->stream);
+    BD_CUDA(cudaGetLastError());
+    h->target_step += (uint64_t)nsteps;
+    return BD_OK;
+  }
   if (!h->graph1) {
     const bd_status st = build_graphs(h);
     if (st) return st;
@@ -1962,7 +1972,7 @@ BD_API const char* bd_stage_name(bd_handle h, int k) {
 
 BD_API bd_status bd_get_kernels_per_step(bd_handle h, int* n) {
   if (!h || !n) return BD_ERR_INVALID_ARGUMENT;
-  if (h->diffuse_only()) *n = (h->Z > 0 ? 2 : 0) + 2;
+  if (h->diffuse_only()) *n = h->Z > 0 ? 4 : 1;
   else if (h->path() == Path::kResident) *n = 1;
   // binned: k_bin, k_scan, k_pairs_cells, k_pairs_big, k_match (+ k_bin_surface
   // with panels); compact: k_count, k_scan, k_scatter, k_pairs_cells,

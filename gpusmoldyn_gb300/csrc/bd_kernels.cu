@@ -527,6 +527,60 @@ __global__ void __launch_bounds__(1024) k_match(KParams p) {
   match_commit<kSurf>(p, c, K, mine, grid, s_match);
 }
 
+// Nothing in a diffusion-only step depends on another record, so a record
+// takes all its steps in registers: one read and one write whatever their
+// number, one launch, and no k_finalize_inplace (the last CTA to finish
+// commits).  Bound by the issue of Philox and Box-Muller: 16 steps of 1M
+// records, with the caller's call, wait and copy of the records, took 297 us
+// as 32 launches and take 155 us; the memory floor is 5 us.  Same operations
+// in the same order as advance_rec, so the same bits.  Without zeroth-order
+// reactions; with them the slot count changes every step.
+template <bool kTable>
+__global__ void __launch_bounds__(256) k_diffuse_steps(KParams p, uint32_t nsteps) {
+  DevCtrl* c = p.ctrl;
+  if (ctrl_status_warp(c)) return;
+  const uint32_t n = ld_u32(&c->n_slots), cur = ld_u32(&c->cur);
+  const uint32_t flags = ld_u32(&p.inst_flags[0]), step0 = ld_u32(&p.inst_step[0]), base = ld_u32(&p.inst_slot_base[0]);
+  const uint32_t target = ld_u32(&p.inst_target[0]);
+  // the instance freezes at its target, and takes a step if it has not yet
+  const uint32_t take = advancing(flags) ? min(nsteps, max(target, step0 + 1u) - step0) : 0u;
+  float4* st = cur ? p.state[1] : p.state[0];
+  const DevInstance& I = p.inst0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    float4 r = st[i];
+    const uint32_t w = rec_w(r);
+    if (w == kDead || take == 0) continue;
+    const float sigma = __ldg(&p.species[I.block * p.S + (w & kSpeciesMask)].sigma);
+    for (uint32_t k = 0; k < take; ++k) {
+      const U4 rn = philox(U4{i - base, step0 + k, kTagDiffuse, 0u}, I.key_lo, I.key_hi);
+      float g0, g1, g2;
+      normals3<kTable>(rn, p.gauss, g0, g1, g2);
+      r.x = reflect(__fmaf_rn(sigma, g0, r.x), I.lo[0], I.hi[0]);
+      r.y = reflect(__fmaf_rn(sigma, g1, r.y), I.lo[1], I.hi[1]);
+      r.z = reflect(__fmaf_rn(sigma, g2, r.z), I.lo[2], I.hi[2]);
+    }
+    st[i] = r;
+  }
+  // every CTA has read the control words before the last one commits
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  __threadfence();
+  if (atomicAdd(&c->bar_count, 1u) != gridDim.x - 1u) return;
+  c->bar_count = 0u;
+  if (take) {
+    p.inst_step[0] = step0 + take;
+    if (step0 + take >= target) {
+      p.inst_flags[0] = flags | kInstFrozen;
+      p.inst_frozen[0] = (uint32_t)c->step + take - 1u;
+    }
+  }
+  c->n_virtual = 0;
+  c->n_pairs_last = 0;
+  c->deaths_last = 0;
+  c->step += nsteps;
+  c->steps_done += nsteps;
+}
+
 template <bool kTable>
 __global__ void __launch_bounds__(256) k_diffuse(KParams p) {
   const DevCtrl* c = p.ctrl;
@@ -727,6 +781,14 @@ void launch_scan(const KParams& p, const LaunchShape& shape, cudaStream_t s) {
   cudaLaunchKernelEx(&cfg, k_scan, p);
 }
 
+void enqueue_diffuse(const KParams& p, bool table, uint32_t nsteps, uint64_t n_slots, cudaStream_t s) {
+  // a record per thread: the work of a record is long and the same for all
+  const uint64_t ctas = (n_slots + 255u) / 256u;
+  const unsigned grid = (unsigned)std::min<uint64_t>(std::max<uint64_t>(ctas, 1u), 1u << 20);
+  if (table) k_diffuse_steps<true><<<grid, 256, 0, s>>>(p, nsteps);
+  else k_diffuse_steps<false><<<grid, 256, 0, s>>>(p, nsteps);
+}
+
 int enqueue_step(const KParams& p, Path path, bool table, bool has_zero, bool has_uni, bool has_bim,
                  const LaunchShape& shape, cudaStream_t s, StageHook hook, void* ctx) {
   (void)has_uni;
@@ -741,6 +803,11 @@ int enqueue_step(const KParams& p, Path path, bool table, bool has_zero, bool ha
     done("k_zeroth");
   }
   if (path == Path::kDiffuseOnly) {
+    if (!has_zero) {
+      enqueue_diffuse(p, table, 1, p.capacity, s);
+      done("k_diffuse_steps");
+      return n;
+    }
     if (table) k_diffuse<true><<<gs, bs, 0, s>>>(p);
     else k_diffuse<false><<<gs, bs, 0, s>>>(p);
     done("k_diffuse");

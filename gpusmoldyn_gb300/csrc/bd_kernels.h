@@ -93,6 +93,8 @@ int resident_grid(int n_sm);
 // short enough to let other streams in.  Most reactions of its one-instance
 // variant.
 constexpr uint32_t kResidentSteps = 64, kResidentReactions = 128;
+// Most steps of one launch of k_diffuse_steps.
+constexpr uint32_t kDiffuseSteps = 64;
 
 // Called after each kernel of a step is enqueued (stage name); lets the
 // profiler record an event between kernels.  nullptr = no callback.
@@ -107,6 +109,10 @@ int enqueue_step(const KParams& p, Path path, bool table, bool has_zero, bool ha
 // launch of k_resident.
 void enqueue_resident(const KParams& p, bool table, bool has_bim, uint32_t nsteps, uint64_t n_slots,
                       const LaunchShape& shape, cudaStream_t stream);
+
+// nsteps steps of a diffusion-only system without zeroth-order reactions and
+// at most n_slots slots, in one launch.
+void enqueue_diffuse(const KParams& p, bool table, uint32_t nsteps, uint64_t n_slots, cudaStream_t stream);
 
 // Count live records per instance (counts[I] must be zeroed).
 void enqueue_instance_counts(const KParams& p, unsigned long long* counts, cudaStream_t stream);
