@@ -153,7 +153,9 @@ struct bd_system {
   float cell_override = 0.0f;
 
   cudaGraphExec_t graph1 = nullptr, graphN = nullptr;
-  KParams graph_params{};     // what the graphs in hand were captured with
+  cudaEvent_t order[2] = {nullptr, nullptr};  // bd_step_async: after the caller's work, after the steps
+  bool graph1_fresh = false, graphN_fresh = false;  // captured with the parameters below
+  KParams graph_params{};     // what the graphs are captured with
   LaunchShape graph_shape{};
   Path graph_path = Path::kBinned;
   LaunchShape shape{};
@@ -267,35 +269,56 @@ KParams make_params(bd_system* h) {
   return p;
 }
 
-bd_status build_graphs(bd_system* h) {
-  const KParams p = make_params(h);
-  const bool table = h->cfg.normal_mode == BD_NORMALS_TABLE;
-  const Path path = h->path();
-  // the graphs capture the parameter block, the launch shape and the path:
-  // when none of them changed (a new upload into the same buffers), the
-  // graphs in hand are still right
-  if (h->graph1 && h->graphN && path == h->graph_path && memcmp(&p, &h->graph_params, sizeof p) == 0 &&
-      memcmp(&h->shape, &h->graph_shape, sizeof h->shape) == 0)
-    return BD_OK;
-  destroy_graphs(h);
-  if (path == Path::kResident || (path == Path::kDiffuseOnly && h->Z == 0)) return BD_OK;  // launched directly
-  const bool has_zero = h->Z > 0, has_uni = h->U > 0, has_bim = h->B > 0;
-  for (int g = 0; g < 2; g++) {
-    const int nsteps = g == 0 ? 1 : kGraphBatch;
+// The graph of one step, or of kGraphBatch.  A stale one is updated in place
+// when its kernels are the same, which saves the instantiation.
+bd_status step_graph(bd_system* h, bool batch, cudaGraphExec_t* out) {
+  cudaGraphExec_t& exec = batch ? h->graphN : h->graph1;
+  bool& fresh = batch ? h->graphN_fresh : h->graph1_fresh;
+  if (!fresh || !exec) {
     cudaGraph_t graph;
     BD_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < nsteps; k++) enqueue_step(p, path, table, has_zero, has_uni, has_bim, h->shape, h->stream);
+    for (int k = 0; k < (batch ? kGraphBatch : 1); k++)
+      enqueue_step(h->graph_params, h->graph_path, h->cfg.normal_mode == BD_NORMALS_TABLE, h->Z > 0, h->U > 0,
+                   h->B > 0, h->graph_shape, h->stream);
     BD_CUDA(cudaStreamEndCapture(h->stream, &graph));
-    cudaGraphExec_t exec;
-    const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
+    cudaError_t e = cudaErrorUnknown;
+    if (exec) {
+      cudaGraphExecUpdateResultInfo info;
+      e = cudaGraphExecUpdate(exec, graph, &info);
+      if (e != cudaSuccess) {
+        cudaGetLastError();  // another topology: build it anew
+        cudaGraphExecDestroy(exec);
+        exec = nullptr;
+      }
+    }
+    if (e != cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
+    if (e != cudaSuccess) exec = nullptr;
     BD_CUDA(e);
-    (g == 0 ? h->graph1 : h->graphN) = exec;
+    fresh = true;
   }
-  h->graph_params = p;
-  h->graph_shape = h->shape;
-  h->graph_path = path;
+  *out = exec;
   return BD_OK;
+}
+
+// The step graphs capture the parameter block, the launch shape and the
+// path: when none of them changed (a new upload into the same buffers), the
+// graphs in hand are still right.  Else the one-step graph is captured here,
+// the batch's when a bd_step first launches it: a server captures anew at
+// every admission, and never takes a batch.
+bd_status refresh_graphs(bd_system* h) {
+  const KParams p = make_params(h);
+  const Path path = h->path();
+  if (path != h->graph_path || memcmp(&p, &h->graph_params, sizeof p) != 0 ||
+      memcmp(&h->shape, &h->graph_shape, sizeof h->shape) != 0) {
+    h->graph1_fresh = h->graphN_fresh = false;
+    h->graph_params = p;
+    h->graph_shape = h->shape;
+    h->graph_path = path;
+  }
+  if (path == Path::kResident || (path == Path::kDiffuseOnly && h->Z == 0)) return BD_OK;  // launched directly
+  cudaGraphExec_t graph;
+  return step_graph(h, false, &graph);
 }
 
 // Uniform grid of one instance: cells at least 1% wider than the largest
@@ -434,7 +457,9 @@ bd_status create_common(const bd_config* cfg, const bd_instance_desc* inst, int 
 
 template <class T>
 bd_status upload(DevBuf<T>& buf, const std::vector<T>& v, cudaStream_t s) {
-  BD_CUDA(buf.alloc(std::max<size_t>(v.size(), 1)));
+  // grow-only: cudaMalloc and cudaFree wait for the device
+  const size_t count = std::max<size_t>(v.size(), 1);
+  if (!buf.p || buf.n < count) BD_CUDA(buf.alloc(count));
   if (!v.empty()) BD_CUDA(cudaMemcpyAsync(buf.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s));
   return BD_OK;
 }
@@ -715,11 +740,11 @@ bd_status upload_particles(bd_system* h, const float* xyz4, const int* species, 
   if ((st = upload(h->inst_flags, h->h_flags, h->stream)) || (st = upload(h->inst_target, h->h_target, h->stream)) ||
       (st = upload(h->inst_frozen, zeros, h->stream)))
     return st;
-  BD_CUDA(h->zero_off.alloc((size_t)I * h->Z + 1));
+  if (h->zero_off.n < (size_t)I * h->Z + 1) BD_CUDA(h->zero_off.alloc((size_t)I * h->Z + 1));
   BD_CUDA(cudaMemsetAsync(h->zero_off.p, 0, ((size_t)I * h->Z + 1) * sizeof(uint32_t), h->stream));
-  BD_CUDA(h->events.alloc((size_t)I * std::max(h->R, 1)));
+  if (h->events.n < (size_t)I * std::max(h->R, 1)) BD_CUDA(h->events.alloc((size_t)I * std::max(h->R, 1)));
   BD_CUDA(cudaMemsetAsync(h->events.p, 0, (size_t)I * std::max(h->R, 1) * sizeof(unsigned long long), h->stream));
-  BD_CUDA(h->pending.alloc((size_t)I * std::max(h->R, 1)));
+  if (h->pending.n < (size_t)I * std::max(h->R, 1)) BD_CUDA(h->pending.alloc((size_t)I * std::max(h->R, 1)));
   BD_CUDA(cudaMemsetAsync(h->pending.p, 0, (size_t)I * std::max(h->R, 1) * sizeof(unsigned long long), h->stream));
   memset(h->hctrl, 0, sizeof(DevCtrl));
   h->hctrl->n_slots = (uint32_t)n;
@@ -727,7 +752,7 @@ bd_status upload_particles(bd_system* h, const float* xyz4, const int* species, 
   if (st) return st;
   h->have_particles = true;
   h->target_step = 0;
-  return build_graphs(h);
+  return refresh_graphs(h);
 }
 
 }  // namespace
@@ -758,6 +783,8 @@ BD_API bd_status bd_destroy(bd_handle h) {
   if (!h->host_only) cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
   destroy_graphs(h);
+  for (cudaEvent_t e : h->order)
+    if (e) cudaEventDestroy(e);
   h->ctrl.free();
   if (h->hctrl) cudaFreeHost(h->hctrl);
   h->dinst.free();
@@ -989,13 +1016,18 @@ bd_status pack_blocks(bd_system* h) {
   }
   h->hzero = ze;
   if (h->host_only) return BD_OK;
-  std::vector<float> gauss(4096);
-  gauss_quantiles(gauss.data(), 4096);
   bd_status st;
+  if (!h->dgauss.p) {  // a constant table: once per handle, computed once per process (2 to 4 ms)
+    static const std::vector<float> gauss = [] {
+      std::vector<float> v(4096);
+      gauss_quantiles(v.data(), 4096);
+      return v;
+    }();
+    if ((st = upload(h->dgauss, gauss, h->stream))) return st;
+  }
   if ((st = upload(h->dspecies, sp, h->stream)) || (st = upload(h->duni, un, h->stream)) ||
       (st = upload(h->dbim, bi, h->stream)) || (st = upload(h->dzero, ze, h->stream)) ||
-      (st = upload(h->dcdf, cdf, h->stream)) || (st = upload(h->dtable, h->bim_table, h->stream)) ||
-      (st = upload(h->dgauss, gauss, h->stream)))
+      (st = upload(h->dcdf, cdf, h->stream)) || (st = upload(h->dtable, h->bim_table, h->stream)))
     return st;
   if (!h->panels.empty()) {
     std::vector<DevPanel> dp(h->panels.size());
@@ -1240,15 +1272,29 @@ BD_API bd_status bd_step(bd_handle h, int nsteps) {
     h->target_step += (uint64_t)nsteps;
     return BD_OK;
   }
-  if (!h->graph1) {
-    const bd_status st = build_graphs(h);
-    if (st) return st;
+  cudaGraphExec_t graph = nullptr;
+  if (left >= kGraphBatch && !h->graphN_fresh) {
+    // inside a caller's stream capture nothing can be captured: single steps
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    BD_CUDA(cudaStreamIsCapturing(h->stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone)
+      for (const int batch = left / kGraphBatch * kGraphBatch; left > nsteps - batch; left--) {
+        const bd_status st = step_graph(h, false, &graph);
+        if (st) return st;
+        BD_CUDA(cudaGraphLaunch(graph, h->stream));
+      }
   }
   while (left >= kGraphBatch) {
-    BD_CUDA(cudaGraphLaunch(h->graphN, h->stream));
+    const bd_status st = step_graph(h, true, &graph);
+    if (st) return st;
+    BD_CUDA(cudaGraphLaunch(graph, h->stream));
     left -= kGraphBatch;
   }
-  while (left-- > 0) BD_CUDA(cudaGraphLaunch(h->graph1, h->stream));
+  while (left-- > 0) {
+    const bd_status st = step_graph(h, false, &graph);
+    if (st) return st;
+    BD_CUDA(cudaGraphLaunch(graph, h->stream));
+  }
   h->target_step += (uint64_t)nsteps;
   return BD_OK;
 }
@@ -1314,23 +1360,17 @@ BD_API bd_status bd_step_async(bd_handle h, int nsteps, void* stream) {
   if (h->host_only) return BD_ERR_NO_DEVICE;
   BD_CUDA(cudaSetDevice(h->device));
   cudaStream_t caller = (cudaStream_t)stream;
-  cudaEvent_t before, after;
-  BD_CUDA(cudaEventCreateWithFlags(&before, cudaEventDisableTiming));
-  if (!cuda_ok(cudaEventCreateWithFlags(&after, cudaEventDisableTiming), "cudaEventCreate")) {
-    cudaEventDestroy(before);
-    return BD_ERR_CUDA;
-  }
-  bd_status st = BD_OK;
-  if (!cuda_ok(cudaEventRecord(before, caller), "cudaEventRecord") ||
-      !cuda_ok(cudaStreamWaitEvent(h->stream, before, 0), "cudaStreamWaitEvent"))
-    st = BD_ERR_CUDA;
-  if (!st) st = bd_step(h, nsteps);
-  if (!st && (!cuda_ok(cudaEventRecord(after, h->stream), "cudaEventRecord") ||
-              !cuda_ok(cudaStreamWaitEvent(caller, after, 0), "cudaStreamWaitEvent")))
-    st = BD_ERR_CUDA;
-  cudaEventDestroy(before);
-  cudaEventDestroy(after);
-  return st;
+  // the handle's two events, made once (making and dropping them took 20 us a
+  // call); a wait refers to the last record before it, so they can be reused
+  for (cudaEvent_t& e : h->order)
+    if (!e) BD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  BD_CUDA(cudaEventRecord(h->order[0], caller));
+  BD_CUDA(cudaStreamWaitEvent(h->stream, h->order[0], 0));
+  const bd_status st = bd_step(h, nsteps);
+  if (st) return st;
+  BD_CUDA(cudaEventRecord(h->order[1], h->stream));
+  BD_CUDA(cudaStreamWaitEvent(caller, h->order[1], 0));
+  return BD_OK;
 }
 
 BD_API bd_status bd_synchronize(bd_handle h) {
@@ -1392,7 +1432,7 @@ BD_API bd_status bd_synchronize(bd_handle h) {
       c.res_left = 0;
       st = push_ctrl(h);
       if (st) return st;
-      st = build_graphs(h);
+      st = refresh_graphs(h);
       if (st) return st;
     }
     const uint64_t left = h->target_step - c.step;
@@ -1572,10 +1612,10 @@ void release_slots(bd_system* h) {
     }
 }
 
+// One element; v stays in place until the stream has been waited for.
 template <class T>
-bd_status put1(DevBuf<T>& buf, int k, T v, cudaStream_t s) {
+bd_status put1(DevBuf<T>& buf, int k, const T& v, cudaStream_t s) {
   BD_CUDA(cudaMemcpyAsync(buf.p + k, &v, sizeof(T), cudaMemcpyHostToDevice, s));
-  BD_CUDA(cudaStreamSynchronize(s));
   return BD_OK;
 }
 
@@ -1660,10 +1700,10 @@ BD_API bd_status bd_instance_admit(bd_handle h, const bd_instance_desc* d, const
         (st = upload(h->inst_flags, h->h_flags, h->stream)) || (st = upload(h->inst_target, h->h_target, h->stream)) ||
         (st = upload(h->inst_frozen, zeros, h->stream)))
       return st;
-    BD_CUDA(h->zero_off.alloc((size_t)I * h->Z + 1));
+    if (h->zero_off.n < (size_t)I * h->Z + 1) BD_CUDA(h->zero_off.alloc((size_t)I * h->Z + 1));
     BD_CUDA(cudaMemsetAsync(h->zero_off.p, 0, ((size_t)I * h->Z + 1) * sizeof(uint32_t), h->stream));
-    BD_CUDA(h->events.alloc((size_t)I * std::max(h->R, 1)));
-    BD_CUDA(h->pending.alloc((size_t)I * std::max(h->R, 1)));
+    if (h->events.n < (size_t)I * std::max(h->R, 1)) BD_CUDA(h->events.alloc((size_t)I * std::max(h->R, 1)));
+    if (h->pending.n < (size_t)I * std::max(h->R, 1)) BD_CUDA(h->pending.alloc((size_t)I * std::max(h->R, 1)));
     BD_CUDA(cudaMemsetAsync(h->pending.p, 0, h->pending.n * sizeof(unsigned long long), h->stream));
     h->have_particles = true;
     h->target_step = 0;
@@ -1683,12 +1723,13 @@ BD_API bd_status bd_instance_admit(bd_handle h, const bd_instance_desc* d, const
                           std::max(h->R, 1) * sizeof(unsigned long long), h->stream));
   h->h_flags[k] = kInstActive;
   h->h_target[k] = steps;
-  if ((st = put1(h->inst_step, k, 0u, h->stream)) || (st = put1(h->inst_slot_base, k, (uint32_t)n_slots, h->stream)) ||
-      (st = put1(h->inst_flags, k, (uint32_t)kInstActive, h->stream)) || (st = put1(h->inst_target, k, steps, h->stream)))
+  const uint32_t words[4] = {0u, (uint32_t)n_slots, kInstActive, steps};  // until push_ctrl has waited
+  if ((st = put1(h->inst_step, k, words[0], h->stream)) || (st = put1(h->inst_slot_base, k, words[1], h->stream)) ||
+      (st = put1(h->inst_flags, k, words[2], h->stream)) || (st = put1(h->inst_target, k, words[3], h->stream)))
     return st;
   h->hctrl->n_slots = (uint32_t)(n_slots + n);
   if ((st = push_ctrl(h))) return st;
-  if ((st = build_graphs(h))) return st;
+  if ((st = refresh_graphs(h))) return st;
   *slot_out = k;
   return BD_OK;
 }
@@ -1784,6 +1825,7 @@ BD_API bd_status bd_instance_harvest(bd_handle h, int k, float* xyz4, int* speci
     *n = total;
     h->h_flags[k] = f[k] | kInstRemoved;
     if ((st = put1(h->inst_flags, k, h->h_flags[k], h->stream))) return st;
+    BD_CUDA(cudaStreamSynchronize(h->stream));
     h->slot_free_after[k] = h->hctrl->step;
     return BD_OK;
   }
@@ -1809,6 +1851,7 @@ BD_API bd_status bd_instance_harvest(bd_handle h, int k, float* xyz4, int* speci
   *n = m;
   h->h_flags[k] = f[k] | kInstRemoved;
   if ((st = put1(h->inst_flags, k, h->h_flags[k], h->stream))) return st;
+  BD_CUDA(cudaStreamSynchronize(h->stream));
   h->slot_free_after[k] = h->hctrl->step;
   return BD_OK;
 }
@@ -1824,6 +1867,7 @@ BD_API bd_status bd_instance_cancel(bd_handle h, int k) {
   BD_CUDA(cudaMemcpy(&f, h->inst_flags.p + k, sizeof(uint32_t), cudaMemcpyDeviceToHost));
   h->h_flags[k] = f | kInstRemoved;
   if ((st = put1(h->inst_flags, k, h->h_flags[k], h->stream))) return st;
+  BD_CUDA(cudaStreamSynchronize(h->stream));
   h->slot_free_after[k] = h->hctrl->step;
   return BD_OK;
 }
@@ -2004,14 +2048,14 @@ BD_API bd_status bd_debug_get_slots(bd_handle h, float* xyz4, uint32_t* w, size_
 BD_API bd_status bd_debug_withhold_scan(bd_handle h, int on) {
   if (!h) return BD_ERR_INVALID_ARGUMENT;
   h->scan_withhold = on != 0;
-  if (h->graph1 || h->graphN) return build_graphs(h);
+  if (h->have_particles) return refresh_graphs(h);
   return BD_OK;
 }
 
 BD_API bd_status bd_debug_withhold_match(bd_handle h, int on) {
   if (!h) return BD_ERR_INVALID_ARGUMENT;
   h->match_withhold = on != 0;
-  if (h->graph1 || h->graphN) return build_graphs(h);
+  if (h->have_particles) return refresh_graphs(h);
   return BD_OK;
 }
 
@@ -2095,7 +2139,7 @@ BD_API bd_status bd_set_launch_shape(bd_handle h, int bs, int cs, int bp, int cp
   if (h->host_only || !h->have_particles) return BD_OK;
   bd_status st = bd_synchronize(h);
   if (st && st != BD_ERR_EMPTY) return st;
-  return build_graphs(h);
+  return refresh_graphs(h);
 }
 
 BD_API bd_status bd_set_cell_size(bd_handle h, float cell_size) {
@@ -2266,9 +2310,9 @@ BD_API bd_status bd_load_checkpoint(bd_handle h, const char* path) {
       (st = upload(h->inst_flags, flags, h->stream)) || (st = upload(h->inst_target, target, h->stream)) ||
       (st = upload(h->inst_frozen, zeros, h->stream)) || (st = upload(h->events, events, h->stream)))
     return st;
-  BD_CUDA(h->zero_off.alloc((size_t)I * h->Z + 1));
+  if (h->zero_off.n < (size_t)I * h->Z + 1) BD_CUDA(h->zero_off.alloc((size_t)I * h->Z + 1));
   BD_CUDA(cudaMemsetAsync(h->zero_off.p, 0, ((size_t)I * h->Z + 1) * sizeof(uint32_t), h->stream));
-  BD_CUDA(h->pending.alloc((size_t)I * std::max(h->R, 1)));
+  if (h->pending.n < (size_t)I * std::max(h->R, 1)) BD_CUDA(h->pending.alloc((size_t)I * std::max(h->R, 1)));
   BD_CUDA(cudaMemsetAsync(h->pending.p, 0, h->pending.n * sizeof(unsigned long long), h->stream));
   memset(h->hctrl, 0, sizeof(DevCtrl));
   h->hctrl->n_slots = (uint32_t)n_slots;
@@ -2278,7 +2322,7 @@ BD_API bd_status bd_load_checkpoint(bd_handle h, const char* path) {
   BD_CUDA(cudaStreamSynchronize(h->stream));
   h->have_particles = true;
   h->target_step = head[1];
-  return build_graphs(h);
+  return refresh_graphs(h);
 }
 
 BD_API bd_status bd_get_config(bd_handle h, bd_config* out) {
