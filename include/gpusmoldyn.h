@@ -373,7 +373,7 @@ BD_API bd_status bd_instance_state(bd_handle h, int slot, uint32_t *steps, uint3
  * d_in, d_out and d_cell_start must be disjoint (an overlap returns
  * BD_ERR_INVALID_ARGUMENT): the kernels read the input while they write the
  * outputs.  Ordering inside a cell is bounded work: a cell of up to 32
- * records costs one thread at most 496 comparisons, a larger cell is sorted
+ * records costs each of them at most 31 comparisons, a larger cell is sorted
  * by one thread block with a bitonic network, O(m log^2 m) for m records.
  * The first call on a device (and the first after a device reset, which
  * reloads the module) looks up that array's device address
