@@ -36,8 +36,10 @@ constexpr int kGraphBatch = 16;
 // and as a chain of kernels (us): 1,000 particles 10.4 / 23.6, 100,000 23.5 /
 // 32.2, 1M (333,333 cells) 54.2 / 56.0, 1.2M 59.7 / 60.3, 2M 90.9 / 83.9.
 constexpr uint32_t kResidentCells = 400000;
-// Mean zeroth-order births per step up to which it does.
-constexpr double kResidentBirths = 4096.0;
+// Mean zeroth-order births per step that one CTA counts and bins beside the
+// others' records (k_resident, k_bin); more are counted by k_zeroth and dealt
+// out over the grid.
+constexpr double kFewBirths = 4096.0;
 // Largest bin array the automatic sort mode accepts.
 constexpr uint64_t kBinBudgetBytes = 32ull << 30;
 
@@ -181,7 +183,7 @@ struct bd_system {
   // outweigh the work.
   double births = 0.0;  // mean zeroth-order births per step
   bool resident() const {
-    return binned && panels.empty() && n_cells <= kResidentCells && births <= kResidentBirths && shape.grid_resident > 0;
+    return binned && panels.empty() && n_cells <= kResidentCells && births <= kFewBirths && shape.grid_resident > 0;
   }
   Path path() const {
     return diffuse_only() ? Path::kDiffuseOnly
@@ -211,7 +213,13 @@ KParams make_params(bd_system* h) {
   p.big_scratch_cap = h->big_scratch.n;
   p.ctrl = h->ctrl.p;
   p.inst = h->dinst.p;
-  if (!h->hinst.empty()) p.inst0 = h->hinst[0];
+  if (!h->hinst.empty()) {
+    p.inst0 = h->hinst[0];
+    for (uint32_t r = 0; r < 10; r++) {
+      p.keys0[2 * r] = p.inst0.key_lo + r * 0x9E3779B9u;
+      p.keys0[2 * r + 1] = p.inst0.key_hi + r * 0xBB67AE85u;
+    }
+  }
   p.species = h->dspecies.p;
   p.uni = h->duni.p;
   p.bim = h->dbim.p;
@@ -230,6 +238,7 @@ KParams make_params(bd_system* h) {
   p.inst_frozen = h->inst_frozen.p;
   p.inst_slot_base = h->inst_slot_base.p;
   p.zero_off = h->zero_off.p;
+  p.births_in_bin = h->Z > 0 && h->births <= kFewBirths ? 1u : 0u;
   p.cell_count = h->cell_count.p;
   p.count_stride = h->count_stride;
   p.cell_start = h->cell_start.p;
@@ -2021,7 +2030,7 @@ BD_API bd_status bd_get_kernels_per_step(bd_handle h, int* n) {
   // binned: k_bin, k_scan, k_pairs_cells, k_pairs_big, k_match (+ k_bin_surface
   // with panels); compact: k_count, k_scan, k_scatter, k_pairs_cells,
   // k_pairs_big, k_match; k_zeroth first with zeroth-order reactions
-  else *n = (h->Z > 0 ? 1 : 0) + (h->binned ? 5 : 6) + (h->binned && !h->panels.empty() ? 1 : 0);
+  else *n = (h->Z > 0 && !(h->binned && h->births <= kFewBirths) ? 1 : 0) + (h->binned ? 5 : 6) + (h->binned && !h->panels.empty() ? 1 : 0);
   return BD_OK;
 }
 

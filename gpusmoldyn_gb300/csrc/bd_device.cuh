@@ -39,6 +39,21 @@ __device__ __forceinline__ U4 philox(U4 c, uint32_t k0, uint32_t k1) {
   return c;
 }
 
+// The same with the ten round keys laid out (k0 and k1 of round r at 2r and
+// 2r + 1): read from the kernel parameters they are constant operands, not
+// additions.
+constexpr int kPhiloxKeys = 20;
+__device__ __forceinline__ U4 philox_keys(U4 c, const uint32_t (&keys)[kPhiloxKeys]) {
+#pragma unroll
+  for (int r = 0; r < 10; ++r) {
+    const uint64_t p0 = (uint64_t)0xD2511F53u * c.x;
+    const uint64_t p1 = (uint64_t)0xCD9E8D57u * c.z;
+    c = U4{(uint32_t)(p1 >> 32) ^ c.y ^ keys[2 * r], (uint32_t)p1, (uint32_t)(p0 >> 32) ^ c.w ^ keys[2 * r + 1],
+           (uint32_t)p0};
+  }
+  return c;
+}
+
 // The reference's randReal: a 32-bit word scaled by 2^-32 in float
 // (rand_kernel.cuh:32-36).  May round to 1.0f, which no coin accepts.
 __device__ __forceinline__ float u32_to_unit(uint32_t v) {
@@ -154,11 +169,18 @@ __device__ __forceinline__ int cell_coord(float x, float lo, float inv, uint32_t
   return c;
 }
 
+// The same for x >= lo: the product is not negative, so its floor is the
+// conversion and needs no lower bound.
+__device__ __forceinline__ uint32_t cell_coord_in_box(float x, float lo, float inv, uint32_t n) {
+  return min(__float2uint_rz(__fmul_rn(__fsub_rn(x, lo), inv)), n - 1u);
+}
+
+// Cell of a position in its instance's box.
 __device__ __forceinline__ uint32_t cell_key(const DevInstance& I, float x, float y, float z) {
-  const int cx = cell_coord(x, I.lo[0], I.inv[0], I.dims[0]);
-  const int cy = cell_coord(y, I.lo[1], I.inv[1], I.dims[1]);
-  const int cz = cell_coord(z, I.lo[2], I.inv[2], I.dims[2]);
-  return I.cell_base + ((uint32_t)cz * I.dims[1] + (uint32_t)cy) * I.dims[0] + (uint32_t)cx;
+  const uint32_t cx = cell_coord_in_box(x, I.lo[0], I.inv[0], I.dims[0]);
+  const uint32_t cy = cell_coord_in_box(y, I.lo[1], I.inv[1], I.dims[1]);
+  const uint32_t cz = cell_coord_in_box(z, I.lo[2], I.inv[2], I.dims[2]);
+  return I.cell_base + (cz * I.dims[1] + cy) * I.dims[0] + cx;
 }
 
 __device__ __forceinline__ uint32_t rec_w(const float4& r) { return __float_as_uint(r.w); }

@@ -237,8 +237,32 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_scatter(KParams p) {
   });
 }
 
+template <bool kSingle>
+__device__ __noinline__ void bin_births(const KParams& p, DevCtrl* c, const SingleCtx& ctx, uint32_t n) {
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t v0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); v0 < n; v0 += stride) {  // whole warps
+    const uint32_t v = v0 + lane_id();
+    Out2 o;
+    o.n = 0;
+    if (v < n) advance_virtual<kSingle>(p, ctx, v, o);
+    claim_retire(p, c, claim_issue(p.cell_count, o.n > 0 ? o.key[0] : kNoKey, o.r[0]));
+    if (__any_sync(kFull, o.n > 1)) claim_retire(p, c, claim_issue(p.cell_count, o.n > 1 ? o.key[1] : kNoKey, o.r[1]));
+  }
+}
+
+// Bound by issue (58% of the slots) and the latency of its loads and atomics
+// at 32 warps per SM; what it does per record is what it costs.  16M c3 step:
+// 227 us -> 202 by taking out of the record's path what rarely applies (the
+// first-order loop behind a bound on the coin's word, one in-box test for the
+// three axes, no lower cell bound, births) and what can be laid out (Philox
+// round keys).  Advancing the few records that react in a call instead, to
+// free registers for a fifth CTA per SM, was slower (219 us at four CTAs, 269
+// at five: the call's conventions spill the loop).
+// Births: those k_zeroth counted, dealt out over the grid; with
+// births_in_bin the last CTA counts and bins them itself, after its records
+// (no k_zeroth: one launch of 4 us less).
 template <bool kTable, int kMinBlocks, bool kSingle, int kSurf = 0>
-__global__ void __launch_bounds__(256, kMinBlocks) k_bin(KParams p) {
+__global__ void __launch_bounds__(256, kMinBlocks) k_bin(const __grid_constant__ KParams p) {
   __shared__ DevSpecies s_species[kSingle ? kCtxSpecies : 1];
   __shared__ DevUni s_uni[kSingle ? kCtxUni : 1];
   __shared__ DeferBuffer s_defer[kSurf == 2 ? 8 : 1];  // one per warp (blocks of at most 256 threads)
@@ -249,8 +273,13 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_bin(KParams p) {
   if (ctrl_status_warp(c)) return;
   const uint32_t cur = ld_u32(&c->cur);
   const float4* __restrict__ st = cur_state(p, cur);
-  const uint32_t n_real = ld_u32(&c->n_slots), n_total = n_real + ld_u32(&c->n_virtual);
-  bin_records<kTable, kSingle, kSurf, false>(p, c, ctx, defer_buf, st, n_real, n_total, p.cell_count);
+  const uint32_t n_real = ld_u32(&c->n_slots);
+  bin_records<kTable, kSingle, kSurf, false>(p, c, ctx, defer_buf, st, n_real, p.cell_count);
+  if (p.births_in_bin) {
+    if (blockIdx.x == gridDim.x - 1u) zeroth_births<kSingle>(p, c, ctx, p.cell_count);
+  } else if (p.Z) {
+    bin_births<kSingle>(p, c, ctx, ld_u32(&c->n_virtual));
+  }
 }
 
 // Binned path with surfaces, pass 1b: the records k_bin queued because
@@ -798,7 +827,7 @@ int enqueue_step(const KParams& p, Path path, bool table, bool has_zero, bool ha
     ++n;
     if (hook) hook(ctx, name);
   };
-  if (has_zero) {
+  if (has_zero && !(path == Path::kBinned && p.births_in_bin)) {
     k_zeroth<<<1, 1024, 0, s>>>(p, path == Path::kDiffuseOnly ? 1 : 0);
     done("k_zeroth");
   }

@@ -15,6 +15,7 @@ struct KParams {
   DevCtrl* ctrl;
   const DevInstance* inst;
   DevInstance inst0;          // copy of instance 0 (kernels specialised for one instance)
+  uint32_t keys0[20];         // its Philox round keys (philox_keys)
   const DevSpecies* species;  // [block][S]
   const DevUni* uni;          // [block][U]
   const DevBim* bim;          // [block][B]
@@ -28,6 +29,7 @@ struct KParams {
   uint32_t* inst_frozen;      // [I] global step (low 32 bits) at which an instance froze
   uint32_t* inst_slot_base;   // [I] first slot of each instance in the current state
   uint32_t* zero_off;         // [I*Z + 1] prefix of zeroth-order births
+  uint32_t births_in_bin;     // k_bin counts the births itself (no k_zeroth)
   DevZero zero0[4];           // instance 0's zeroth-order entries when Z <= 4 (k_zeroth's one-instance path)
   uint32_t* cell_count;       // [n_cells] particles per cell (returns to 0 each step)
   uint32_t count_stride;      // words to the second count array (k_resident alternates between them)

@@ -85,7 +85,7 @@ enum InstanceFlags : uint32_t {
   kInstRemoved = 4u,       // dropped at the next sort
 };
 
-struct DevInstance {       // 80 B
+struct DevInstance {       // 80 B (rows of the instance table start on 16 bytes)
   float lo[3], hi[3];      // reflecting box
   float inv[3];            // cells per unit length per axis
   float cell[3];           // cell edge per axis

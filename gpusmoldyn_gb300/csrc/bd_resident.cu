@@ -122,35 +122,6 @@ __device__ __forceinline__ void leave(DevCtrl* c) {
   }
 }
 
-// Exclusive scan over the CTA's threads; *total the sum, in every thread.
-__device__ __forceinline__ uint32_t cta_scan(uint32_t v, uint32_t* total) {
-  __shared__ uint32_t s_sum[kWarps], s_total;
-  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-  uint32_t incl = v;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t n = __shfl_up_sync(kFull, incl, d);
-    if (lane >= (uint32_t)d) incl += n;
-  }
-  __syncthreads();  // s_sum and s_total of the last call are no longer read
-  if (lane == 31) s_sum[warp] = incl;
-  __syncthreads();
-  if (warp == 0) {
-    const uint32_t x = s_sum[lane];
-    uint32_t y = x;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t n = __shfl_up_sync(kFull, y, d);
-      if (lane >= (uint32_t)d) y += n;
-    }
-    s_sum[lane] = y - x;
-    if (lane == 31) s_total = y;
-  }
-  __syncthreads();
-  *total = s_total;
-  return s_sum[warp] + incl - v;
-}
-
 // Counts [lo, hi) (lo a multiple of 4, hi - lo <= kSmallCells) scanned by the
 // CTA into s[0, hi - lo]: s[i] = the counts of the first i cells.  Returns
 // their sum.  Loads are 16 bytes a thread and all in flight together; each
@@ -176,50 +147,6 @@ __device__ __forceinline__ uint32_t scan_counts(const uint32_t* counts, uint32_t
   if (threadIdx.x == kThreads - 1u) s[n] = total;
   __syncthreads();
   return total;
-}
-
-// Zeroth-order births of the step, counted (inversion of the Poisson CDFs, as
-// k_zeroth) and binned by one CTA while the others advance the records.
-template <bool kSingle>
-__device__ __noinline__ void zeroth_births(const KParams& p, DevCtrl* c, const SingleCtx& ctx, uint32_t* counts) {
-  const uint32_t nz = p.n_inst * p.Z;
-  uint32_t carry = 0;
-  for (uint32_t base = 0; base < nz; base += kThreads) {
-    const uint32_t e = base + threadIdx.x;
-    uint32_t cnt = 0;
-    if (e < nz) {
-      const uint32_t inst = e / p.Z, zr = e % p.Z;
-      const DevInstance& I = inst_of<kSingle>(p, inst);
-      if (advancing(kSingle ? ctx.flags : p.inst_flags[inst])) {
-        const DevZero& Zr = p.zero[I.block * p.Z + zr];
-        const U4 r = philox(U4{zr, kSingle ? ctx.step : p.inst_step[inst], kTagZeroCount, 0u}, I.key_lo, I.key_hi);
-        const double u = u53_to_unit(r.x, r.y);
-        const double* cdf = p.cdf + Zr.cdf_off;
-        uint32_t lo = 0, hi = Zr.cdf_len - 1;
-        while (lo < hi) {
-          const uint32_t mid = (lo + hi) >> 1;
-          if (cdf[mid] > u) hi = mid;
-          else lo = mid + 1;
-        }
-        cnt = (uint32_t)Zr.kmin + lo;
-        if (cnt) atomicAdd(&p.pending[(size_t)inst * p.R + Zr.rxn], (unsigned long long)cnt);
-      }
-    }
-    uint32_t total;
-    const uint32_t ex = cta_scan(cnt, &total);
-    if (e < nz) p.zero_off[e] = carry + ex;
-    carry += total;
-  }
-  if (threadIdx.x == 0) p.zero_off[nz] = carry;
-  __syncthreads();
-  for (uint32_t v0 = threadIdx.x & ~31u; v0 < carry; v0 += kThreads) {  // whole warps
-    const uint32_t v = v0 + lane_id();
-    Out2 o;
-    o.n = 0;
-    if (v < carry) advance_virtual<kSingle>(p, ctx, v, o);
-    claim_retire(p, c, claim_issue(counts, o.n > 0 ? o.key[0] : kNoKey, o.r[0]));
-    if (__any_sync(kFull, o.n > 1)) claim_retire(p, c, claim_issue(counts, o.n > 1 ? o.key[1] : kNoKey, o.r[1]));
-  }
 }
 
 // The parts that few steps reach, or that one CTA runs, are calls: inlined,
@@ -283,7 +210,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident(const __grid_constant_
   for (uint32_t k = 0; k < nsteps; ++k) {
     uint32_t* counts = p.cell_count + (step & 1u) * (size_t)p.count_stride;
     uint32_t* other = p.cell_count + (~step & 1u) * (size_t)p.count_stride;
-    bin_records<kTable, kSingle, 0, true>(p, c, ctx, s_defer, cur_state(p, cur), n_real, n_real, counts);
+    bin_records<kTable, kSingle, 0, true>(p, c, ctx, s_defer, cur_state(p, cur), n_real, counts);
     if (p.Z && blockIdx.x == gridDim.x - 1u) zeroth_births<kSingle>(s_params, c, ctx, counts);
     if (p.scan_withhold && blockIdx.x == 0) {  // test switch: CTA 0 never arrives
       if (gridDim.x == 1 && threadIdx.x == 0) atomicOr(&c->status, kStatTimeout);

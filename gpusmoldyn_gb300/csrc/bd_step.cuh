@@ -133,7 +133,10 @@ __device__ __forceinline__ uint32_t word_of(const U4& c, uint32_t k) {
 template <bool kSingle>
 __device__ __forceinline__ const DevInstance& inst_of(const KParams& p, uint32_t inst) {
   if (kSingle) return p.inst0;
-  return p.inst[inst];
+  // rows of 80 bytes: fields side by side come in one load (64 c4 instances:
+  // k_pairs_cells 194.8 -> 190.2 us)
+  static_assert(sizeof(DevInstance) % 16 == 0, "16-byte rows");
+  return *static_cast<const DevInstance*>(__builtin_assume_aligned(&p.inst[inst], 16));
 }
 
 // What every record of a one-instance handle reads, loaded once per CTA:
@@ -147,9 +150,24 @@ struct SingleCtx {
   const DevUni* uni;
 };
 
-// Fills the shared tables (all threads of the CTA call it; one barrier).
+// A word above it cannot be accepted as the coin of the species' only
+// first-order reaction (u32_to_unit rounds by at most 128); 0 without one,
+// all ones with several, whose other coins have to be drawn.
+__device__ __forceinline__ uint32_t first_coin_bound(const DevSpecies& s, const DevUni* uni) {
+  if (s.uni_count != 1u) return s.uni_count ? 0xFFFFFFFFu : 0u;
+  const double bound = (double)uni[s.uni_begin].prob * 4294967296.0 + 256.0;
+  return bound < 4294967295.0 ? (uint32_t)bound : 0xFFFFFFFFu;
+}
+
+// Fills the shared tables (all threads of the CTA call it; one barrier).  The
+// species' max_r, which the advance does not need, holds the bits of
+// first_coin_bound.
 __device__ __forceinline__ SingleCtx single_ctx(const KParams& p, DevSpecies* s_species, DevUni* s_uni) {
-  for (uint32_t t = threadIdx.x; t < p.S; t += blockDim.x) s_species[t] = p.species[t];
+  for (uint32_t t = threadIdx.x; t < p.S; t += blockDim.x) {
+    DevSpecies s = p.species[t];
+    s.max_r = __uint_as_float(first_coin_bound(s, p.uni));
+    s_species[t] = s;
+  }
   for (uint32_t t = threadIdx.x; t < p.U; t += blockDim.x) s_uni[t] = p.uni[t];
   __syncthreads();
   return SingleCtx{ld_u32(&p.inst_flags[0]), ld_u32(&p.inst_step[0]), ld_u32(&p.inst_slot_base[0]), s_species,
@@ -191,8 +209,8 @@ __device__ __forceinline__ void advance_rec(const KParams& p, const SingleCtx& c
   const uint32_t inst = w >> 16, sp = w & kSpeciesMask;
   const DevInstance& I = inst_of<kSingle>(p, inst);
   const uint32_t flags = kSingle ? ctx.flags : p.inst_flags[inst];
-  if (flags & kInstRemoved) return;
-  if ((flags & kInstFrozen) || !(flags & kInstActive)) {
+  if (!advancing(flags)) {  // frozen or not active: kept where it is
+    if (flags & kInstRemoved) return;
     o.r[0] = rec;
     o.key[0] = cell_key(I, rec.x, rec.y, rec.z);
     o.n = 1;
@@ -206,12 +224,17 @@ __device__ __forceinline__ void advance_rec(const KParams& p, const SingleCtx& c
   // arithmetic that hides its latency
   const uint32_t near = kSurf == 2 ? __ldg(&p.cell_surf[cell_key(I, rec.x, rec.y, rec.z)]) : 0u;
 
-  const U4 rn = philox(U4{local, t, kTagDiffuse, 0u}, k0, k1);
+  const U4 rn = kSingle ? philox_keys(U4{local, t, kTagDiffuse, 0u}, p.keys0)
+                        : philox(U4{local, t, kTagDiffuse, 0u}, k0, k1);
   float g0, g1, g2;
   normals3<kTable>(rn, p.gauss, g0, g1, g2);
-  float x = reflect(__fmaf_rn(S.sigma, g0, rec.x), I.lo[0], I.hi[0]);
-  float y = reflect(__fmaf_rn(S.sigma, g1, rec.y), I.lo[1], I.hi[1]);
-  float z = reflect(__fmaf_rn(S.sigma, g2, rec.z), I.lo[2], I.hi[2]);
+  float x = __fmaf_rn(S.sigma, g0, rec.x), y = __fmaf_rn(S.sigma, g1, rec.y), z = __fmaf_rn(S.sigma, g2, rec.z);
+  // one branch for the three axes
+  if (!(x >= I.lo[0] && x <= I.hi[0] && y >= I.lo[1] && y <= I.hi[1] && z >= I.lo[2] && z <= I.hi[2])) {
+    x = reflect(x, I.lo[0], I.hi[0]);
+    y = reflect(y, I.lo[1], I.hi[1]);
+    z = reflect(z, I.lo[2], I.hi[2]);
+  }
   if (kSurf == 2 && ((near >> (sp < 7u ? sp : 7u)) & 1u)) {
     o.n = -1;
     return;
@@ -222,7 +245,9 @@ __device__ __forceinline__ void advance_rec(const KParams& p, const SingleCtx& c
 
   // coin 0 is the diffusion block's spare word; coins 1.. come 4 per block
   U4 coins = rn;
-  for (uint32_t k = 0; k < S.uni_count; ++k) {
+  // most records of a one-instance handle leave by their first word
+  const uint32_t n_uni = !kSingle || rn.w <= __float_as_uint(S.max_r) ? S.uni_count : 0u;
+  for (uint32_t k = 0; k < n_uni; ++k) {
     if (k > 0 && ((k - 1) & 3u) == 0) coins = philox(U4{local, t, kTagUniCoin | ((k - 1) >> 2), 0u}, k0, k1);
     const DevUni& u = kSingle ? ctx.uni[S.uni_begin + k] : p.uni[I.block * p.U + S.uni_begin + k];
     if (u32_to_unit(k == 0 ? rn.w : word_of(coins, k - 1)) < u.prob) {
@@ -401,7 +426,8 @@ __device__ bool grid_barrier(DevCtrl* c) {
 // sectors rather than half of one shared with a neighbour cell.  The pair
 // kernel reads a cell's first kBinGroup places from one group.
 __device__ __forceinline__ size_t bin_index(const KParams& p, uint32_t cell, uint32_t off) {
-  return ((size_t)(off / kBinGroup) * p.n_cells + cell) * kBinGroup + off % kBinGroup;
+  // the group's number fits 32 bits (2^32 groups would be 256 GiB)
+  return (size_t)((off / kBinGroup) * p.n_cells + cell) * kBinGroup + off % kBinGroup;
 }
 
 // A record waiting for its place in a bin: the warp's claim (atomicAdd on
@@ -466,19 +492,17 @@ __device__ __forceinline__ void defer_flush(const KParams& p, DevCtrl* c, DeferB
 
 template <bool kTable, bool kSingle, int kSurf, bool kSpread>
 __device__ __forceinline__ void bin_records(const KParams& p, DevCtrl* c, const SingleCtx& ctx, DeferBuffer& defer_buf,
-                                            const float4* __restrict__ st, uint32_t n_real, uint32_t n_total,
-                                            uint32_t* counts) {
+                                            const float4* __restrict__ st, uint32_t n_real, uint32_t* counts) {
   uint32_t n_defer = 0;  // slots in defer_buf (warp-uniform)
   PendingClaim pending;
   pending.key = kNoKey;
   pending.old = 0;
   pending.leader = 0;
   pending.rank = 0;
-  stream_records<kSpread>(st, n_real, n_total, [&](uint32_t i, const float4& rec) {
+  stream_records<kSpread>(st, n_real, n_real, [&](uint32_t i, const float4& rec) {
     Out2 o;
     o.n = 0;
     if (i < n_real) advance_rec<kTable, true, kSingle, kSurf>(p, ctx, rec, i, o);
-    else if (i < n_total) advance_virtual<kSingle>(p, ctx, i - n_real, o);
     if (kSurf == 2) {
       // records near a panel go to k_bin_surface
       const bool defer = o.n < 0;
@@ -504,6 +528,81 @@ __device__ __forceinline__ void bin_records(const KParams& p, DevCtrl* c, const 
   });
   claim_retire(p, c, pending);
   if (kSurf == 2 && n_defer > 0) defer_flush(p, c, defer_buf, n_defer);
+}
+
+// Exclusive scan over the CTA's threads (whole warps); *total the sum, in
+// every thread.
+__device__ __forceinline__ uint32_t cta_scan(uint32_t v, uint32_t* total) {
+  __shared__ uint32_t s_sum[32], s_total;
+  const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+  uint32_t incl = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t n = __shfl_up_sync(kFull, incl, d);
+    if (lane >= (uint32_t)d) incl += n;
+  }
+  __syncthreads();  // s_sum and s_total of the last call are no longer read
+  if (lane == 31) s_sum[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    const uint32_t x = lane < (blockDim.x >> 5) ? s_sum[lane] : 0u;
+    uint32_t y = x;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t n = __shfl_up_sync(kFull, y, d);
+      if (lane >= (uint32_t)d) y += n;
+    }
+    s_sum[lane] = y - x;
+    if (lane == 31) s_total = y;
+  }
+  __syncthreads();
+  *total = s_total;
+  return s_sum[warp] + incl - v;
+}
+
+// Zeroth-order births of the step, counted (inversion of the Poisson CDFs, as
+// k_zeroth) and binned by one CTA while the others advance the records; a
+// call, so that its registers are not the streaming loop's.
+template <bool kSingle>
+__device__ __noinline__ void zeroth_births(const KParams& p, DevCtrl* c, const SingleCtx& ctx, uint32_t* counts) {
+  const uint32_t nz = p.n_inst * p.Z;
+  uint32_t carry = 0;
+  for (uint32_t base = 0; base < nz; base += blockDim.x) {
+    const uint32_t e = base + threadIdx.x;
+    uint32_t cnt = 0;
+    if (e < nz) {
+      const uint32_t inst = e / p.Z, zr = e % p.Z;
+      const DevInstance& I = inst_of<kSingle>(p, inst);
+      if (advancing(kSingle ? ctx.flags : p.inst_flags[inst])) {
+        const DevZero& Zr = p.zero[I.block * p.Z + zr];
+        const U4 r = philox(U4{zr, kSingle ? ctx.step : p.inst_step[inst], kTagZeroCount, 0u}, I.key_lo, I.key_hi);
+        const double u = u53_to_unit(r.x, r.y);
+        const double* cdf = p.cdf + Zr.cdf_off;
+        uint32_t lo = 0, hi = Zr.cdf_len - 1;
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (cdf[mid] > u) hi = mid;
+          else lo = mid + 1;
+        }
+        cnt = (uint32_t)Zr.kmin + lo;
+        if (cnt) atomicAdd(&p.pending[(size_t)inst * p.R + Zr.rxn], (unsigned long long)cnt);
+      }
+    }
+    uint32_t total;
+    const uint32_t ex = cta_scan(cnt, &total);
+    if (e < nz) p.zero_off[e] = carry + ex;
+    carry += total;
+  }
+  if (threadIdx.x == 0) p.zero_off[nz] = carry;
+  __syncthreads();
+  for (uint32_t v0 = threadIdx.x & ~31u; v0 < carry; v0 += blockDim.x) {  // whole warps
+    const uint32_t v = v0 + lane_id();
+    Out2 o;
+    o.n = 0;
+    if (v < carry) advance_virtual<kSingle>(p, ctx, v, o);
+    claim_retire(p, c, claim_issue(counts, o.n > 0 ? o.key[0] : kNoKey, o.r[0]));
+    if (__any_sync(kFull, o.n > 1)) claim_retire(p, c, claim_issue(counts, o.n > 1 ? o.key[1] : kNoKey, o.r[1]));
+  }
 }
 
 // The records of one cell, m-th at base[(m / kBinGroup) * stride + m %
