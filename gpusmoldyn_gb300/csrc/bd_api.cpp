@@ -132,6 +132,8 @@ struct bd_system {
   DevBuf<double> dcdf;
   DevBuf<int32_t> dtable;
   DevBuf<float> dgauss;
+  DevBuf<float4> dnear_grid, dnear_lim;  // KParams::near_grid, near_lim
+  std::vector<float> max_r;              // [I S] largest binding radii
   DevBuf<uint32_t> inst_step, inst_slot_base, zero_off;
   DevBuf<unsigned long long> events, pending;
   DevBuf<float4> state0, state1, scatter, bins;
@@ -200,6 +202,17 @@ void destroy_graphs(bd_system* h) {
   h->graph1 = h->graphN = nullptr;
 }
 
+constexpr float kPruneMargin = 1e-3f;  // fraction of a cell edge added to pruning distances
+
+// Shift of the pair search's grid coordinate fma(x, inv, shift) along axis a
+// (KParams::near_grid): below -lo inv by more than the rounding of it and of
+// the kernels' own (x - lo) inv, which stays under 2^-21 of the magnitudes
+// that enter.
+double near_margin(const DevInstance& I, int a) {
+  return (fabs((double)I.lo[a] * I.inv[a]) + fabs((double)I.hi[a] * I.inv[a]) + (double)I.dims[a]) * 5e-7 + 1e-6;
+}
+float near_shift(const DevInstance& I, int a) { return (float)(-(double)I.lo[a] * I.inv[a] - near_margin(I, a)); }
+
 KParams make_params(bd_system* h) {
   KParams p{};
   p.state[0] = h->state0.p;
@@ -215,6 +228,7 @@ KParams make_params(bd_system* h) {
   p.inst = h->dinst.p;
   if (!h->hinst.empty()) {
     p.inst0 = h->hinst[0];
+    for (int a = 0; a < 3; a++) p.near_shift[a] = near_shift(p.inst0, a);
     for (uint32_t r = 0; r < 10; r++) {
       p.keys0[2 * r] = p.inst0.key_lo + r * 0x9E3779B9u;
       p.keys0[2 * r + 1] = p.inst0.key_hi + r * 0xBB67AE85u;
@@ -260,7 +274,9 @@ KParams make_params(bd_system* h) {
   p.n_tiles = h->n_tiles;
   p.capacity = (uint32_t)h->capacity;
   p.pair_cap = h->pair_cap;
-  p.prune_margin = 1e-3f;
+  p.prune_margin = kPruneMargin;
+  p.near_grid = h->dnear_grid.p;
+  p.near_lim = h->dnear_lim.p;
   p.n_panels = (uint32_t)h->panels.size();
   if (p.n_panels) {
     p.panels = h->dpanels.p;
@@ -598,6 +614,24 @@ bd_status layout_cells(bd_system* h) {
   BD_CUDA(ensure(h->cell_start, (size_t)h->n_cells + 1));
   BD_CUDA(cudaMemsetAsync(h->cell_start.p, 0, ((size_t)h->n_cells + 1) * sizeof(uint32_t), h->stream));
   BD_CUDA(ensure(h->tile_sums, (size_t)std::max<uint32_t>(h->n_tiles, (uint32_t)std::max(h->shape.grid_resident, 1))));
+  // the pair search's bounds in the new grids
+  std::vector<float4> grid(2 * (size_t)I), lim((size_t)I * h->S);
+  for (int k = 0; k < I; k++) {
+    const DevInstance& D = h->hinst[k];
+    float margin = kPruneMargin * std::min(D.cell[0], std::min(D.cell[1], D.cell[2]));
+    grid[2 * k] = make_float4(D.inv[0], D.inv[1], D.inv[2], 0.0f);
+    grid[2 * k + 1] = make_float4(near_shift(D, 0), near_shift(D, 1), near_shift(D, 2), 0.0f);
+    for (int s = 0; s < h->S; s++) {
+      const float r = h->max_r[(size_t)D.block * h->S + s];
+      float from[3];
+      for (int a = 0; a < 3; a++)
+        from[a] = (float)(1.0 - 1.01 * ((double)r + margin) * D.inv[a] - 2.0 * near_margin(D, a));
+      lim[(size_t)k * h->S + s] = r > 0.0f ? make_float4(r * 1.001f, from[0], from[1], from[2])
+                                           : make_float4(-1.0f, 2.0f, 2.0f, 2.0f);
+    }
+  }
+  bd_status up;
+  if ((up = upload(h->dnear_grid, grid, h->stream)) || (up = upload(h->dnear_lim, lim, h->stream))) return up;
   BD_CUDA(cudaStreamSynchronize(h->stream));
   if (!h->panels.empty()) {
     const bd_status st = upload_cell_masks(h);
@@ -797,6 +831,8 @@ BD_API bd_status bd_destroy(bd_handle h) {
   h->ctrl.free();
   if (h->hctrl) cudaFreeHost(h->hctrl);
   h->dinst.free();
+  h->dnear_grid.free();
+  h->dnear_lim.free();
   h->dspecies.free();
   h->duni.free();
   h->dbim.free();
@@ -1024,6 +1060,8 @@ bd_status pack_blocks(bd_system* h) {
     }
   }
   h->hzero = ze;
+  h->max_r.resize((size_t)I * S);
+  for (size_t k = 0; k < h->max_r.size(); k++) h->max_r[k] = sp[k].max_r;
   if (h->host_only) return BD_OK;
   bd_status st;
   if (!h->dgauss.p) {  // a constant table: once per handle, computed once per process (2 to 4 ms)

@@ -50,6 +50,14 @@ struct KParams {
   float4* big_scratch;        // [big_scratch_cap] sort buffers of k_pairs_big, two of [capacity]
   uint32_t big_cap;
   uint64_t big_scratch_cap;
+  // What the pair search reads per record.  near_grid: [2 I] cells per unit
+  // length and the shift of g = fma(x, inv, shift), the grid coordinate less
+  // more than any rounding of it.  near_lim: [I S] the bound on |dx| and |dy|
+  // of the species' pairs (negative without any) and the fractions of a cell
+  // from which on a record may reach the +x, +y and +z neighbour.
+  const float4* near_grid;
+  const float4* near_lim;
+  float near_shift[3];        // of instance 0
   float prune_margin;         // fraction of a cell edge added to pruning distances
   // surfaces (n_panels = 0: none)
   const DevPanel* panels;     // [n_panels]

@@ -730,22 +730,20 @@ __device__ __forceinline__ void emit(const KParams& p, DevCtrl* c, const uint32_
             inst_of<kSingle>(p, k.inst));
 }
 
-// True when record k may lie within its largest binding radius (plus the
-// pruning margin) of a +x, +y or +z face of its cell, i.e. when
-// forward_mask may return a neighbour; false for most records, which lie
-// deeper inside their cell.  The test runs on the fractional grid
-// coordinates: frac = g - floor(g) is exact (Sterbenz), and the 1% slack
-// exceeds the rounding of forward_mask's face distances, so it never
-// rejects a record that forward_mask would give a neighbour.
-template <bool kSingle>
-__device__ __forceinline__ bool near_forward_face(const KParams& p, const Seeker& k) {
-  const DevInstance& I = inst_of<kSingle>(p, k.inst);
-  const float gx = __fmul_rn(__fsub_rn(k.r.x, I.lo[0]), I.inv[0]);
-  const float gy = __fmul_rn(__fsub_rn(k.r.y, I.lo[1]), I.inv[1]);
-  const float gz = __fmul_rn(__fsub_rn(k.r.z, I.lo[2]), I.inv[2]);
-  const float slack = 1.01f * (k.max_r + p.prune_margin * fminf(I.cell[0], fminf(I.cell[1], I.cell[2])));
-  return !(1.0f - (gx - floorf(gx)) > slack * I.inv[0] && 1.0f - (gy - floorf(gy)) > slack * I.inv[1] &&
-           1.0f - (gz - floorf(gz)) > slack * I.inv[2]);
+// True when a record may lie within its largest binding radius (plus the
+// pruning margin) of a +x, +y or +z face of its cell, i.e. when forward_mask
+// may return a neighbour; false for most records, which lie deeper inside
+// their cell.  inv, shift: of its instance (KParams::near_grid); lim: of its
+// species.  The grid coordinates are shifted down by more than any rounding
+// of them, so none rounds up past the face it is near, and the 1% slack of
+// lim exceeds the rounding of forward_mask's face distances: it never rejects
+// a record that forward_mask would give a neighbour.
+__device__ __forceinline__ bool near_forward_face(const float4& r, const float4& lim, const float (&inv)[3],
+                                                  const float (&shift)[3]) {
+  const float gx = __fmaf_rn(r.x, inv[0], shift[0]);
+  const float gy = __fmaf_rn(r.y, inv[1], shift[1]);
+  const float gz = __fmaf_rn(r.z, inv[2], shift[2]);
+  return gx - floorf(gx) >= lim.y || gy - floorf(gy) >= lim.z || gz - floorf(gz) >= lim.w;
 }
 
 // The forward neighbour cells (higher key) of record k that its largest
@@ -917,36 +915,31 @@ __device__ __forceinline__ void drain_faces(const KParams& p, DevCtrl* c, const 
 }
 
 // Per-species tables of a one-instance handle's pair search: the largest
-// binding radius and the near-face thresholds of near_forward_face in grid
-// units (x, y, z), computed once per CTA with the same operations (0.2412 ->
-// 0.2403 ms on the 16M c3 step).
+// binding radius, and KParams::near_lim.
 template <bool kSingle>
 struct PairSpecies {
   float max_r[kSingle ? kCtxSpecies : 1];
-  float4 near[kSingle ? kCtxSpecies : 1];
+  float4 lim[kSingle ? kCtxSpecies : 1];
 };
 
 // All threads of the CTA call it; one barrier.
 template <bool kSingle>
 __device__ __forceinline__ void pair_species(const KParams& p, PairSpecies<kSingle>& sp) {
-  if constexpr (!kSingle) return;
-  for (uint32_t t = threadIdx.x; kSingle && t < p.S; t += blockDim.x) {
-    const float mr = p.species[p.inst0.block * p.S + t].max_r;
-    sp.max_r[t] = mr;
-    const DevInstance& I = p.inst0;
-    const float slack = 1.01f * (mr + p.prune_margin * fminf(I.cell[0], fminf(I.cell[1], I.cell[2])));
-    sp.near[t] = make_float4(slack * I.inv[0], slack * I.inv[1], slack * I.inv[2], 0.0f);
+  if constexpr (kSingle) {
+    for (uint32_t t = threadIdx.x; t < p.S; t += blockDim.x) {
+      sp.max_r[t] = p.species[p.inst0.block * p.S + t].max_r;
+      sp.lim[t] = p.near_lim[t];
+    }
+    __syncthreads();
   }
-  __syncthreads();
 }
 
 // Per-warp working sets of the pair search (CTAs of kWarps warps): the ring of
-// the open tasks' non-empty cells -- (key, first slot) and (records, stream
-// offset of the cell's first record) -- and the records near a +face.
+// the open tasks' non-empty cells -- key, first slot, records, stream offset of
+// the cell's first record -- and the records near a +face.
 template <bool kHasBim, int kWarps>
 struct PairShared {
-  uint2 cell[kWarps][kCellRing];
-  uint2 meta[kWarps][kCellRing];
+  uint4 cell[kWarps][kCellRing];
   FaceQueue face[kHasBim ? kWarps : 1];
   uint32_t ticket;  // kOwn: tasks of the CTA's range taken
 };
@@ -1037,8 +1030,7 @@ __device__ __forceinline__ void pair_cells(const KParams& p, DevCtrl* c, float4*
       __syncwarp();  // the ring entries about to be replaced are no longer read
       if (n > 0) {
         const uint32_t e = (entries + __popc(ball & ((1u << lane) - 1u))) & (kCellRing - 1u);
-        sh.cell[warp][e] = make_uint2(cell, cs);
-        sh.meta[warp][e] = make_uint2(n, off);
+        sh.cell[warp][e] = make_uint4(cell, cs, n, off);
       }
       entries += __popc(ball);
       last = loaded;
@@ -1058,15 +1050,25 @@ __device__ __forceinline__ void pair_cells(const KParams& p, DevCtrl* c, float4*
     float4 ra = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (t < loaded) {
       const uint32_t e = (before + __popc(M & le_mask) - 1u) & (kCellRing - 1u);
-      const uint2 cc = sh.cell[warp][e];
-      const uint2 meta = sh.meta[warp][e];
-      const uint32_t ocell = cc.x, ocs = cc.y, on = meta.x;
-      const uint32_t j = t - meta.y;
+      const uint4 cc = sh.cell[warp][e];
+      const uint32_t ocell = cc.x, ocs = cc.y, on = cc.z;
+      const uint32_t j = t - cc.w;
       const CellView cb = cell_records<kBinned>(p, ocell, ocs);
-      ra = cb.ldg(j);
-      Seeker k;
-      const bool search = kHasBim && seeker_init<kSingle>(p, ra, k, kSingle ? sp.max_r : nullptr, adv0);
-      const float xlim = search ? k.xlim : -1.0f;
+      ra = kBinned ? ld_step(&p.bins[bin_index(p, ocell, j)]) : cb.ldg(j);
+      // the record's bounds, in one load (two with its instance's flags); its
+      // seeker is made only when it has candidates (k_pairs_cells 234 -> 221.5
+      // us on the 16M c3 step, 190 -> 183 on 64 c4 instances, whose records
+      // loaded 14 words of their instance and species before)
+      float4 lim = make_float4(-1.0f, 2.0f, 2.0f, 2.0f);
+      if (kHasBim && kSingle) {
+        if (adv0 && !(rec_w(ra) & kNewborn)) lim = sp.lim[rec_w(ra) & kSpeciesMask];
+      } else if (kHasBim) {
+        const uint32_t w = rec_w(ra), inst = w >> 16;
+        const bool adv = advancing(ld_step(&p.inst_flags[inst]));
+        const float4 l = __ldg(&p.near_lim[inst * p.S + (w & kSpeciesMask)]);
+        if (adv && !(w & kNewborn)) lim = l;
+      }
+      const float xlim = lim.x;
       const uint32_t rx = __float_as_uint(ra.x);
       // rank: members with smaller x bits; le also counts equal ones (the
       // record itself among them), so le - rank > 1 means a tie to break
@@ -1111,7 +1113,9 @@ __device__ __forceinline__ void pair_cells(const KParams& p, DevCtrl* c, float4*
       ca = ocs + rank;
       if (ca < p.capacity) nx[ca] = make_float4(ra.x, ra.y, ra.z, __uint_as_float(rec_w(ra) & ~kNewborn));
       else raise(c, kStatBounds);
-      if (search) {
+      if (kHasBim && (cand || (on > 32u && xlim >= 0.0f))) {
+        Seeker k;
+        seeker_init<kSingle>(p, ra, k, kSingle ? sp.max_r : nullptr, adv0);
         while (cand) {
           const uint32_t m = (uint32_t)(__ffs(cand) - 1);
           cand &= cand - 1u;
@@ -1124,16 +1128,14 @@ __device__ __forceinline__ void pair_cells(const KParams& p, DevCtrl* c, float4*
           const int32_t bb = pair_reaction(p, k, qm);
           if (bb >= 0) emit<kSingle>(p, c, starts, k, ca, ocs + canonical_rank(cb, 0, on, m, qm), bb);
         }
-        if (kSingle) {
-          const float4 sn = sp.near[rec_w(ra) & kSpeciesMask];
-          const DevInstance& I = p.inst0;
-          const float gx = __fmul_rn(__fsub_rn(ra.x, I.lo[0]), I.inv[0]);
-          const float gy = __fmul_rn(__fsub_rn(ra.y, I.lo[1]), I.inv[1]);
-          const float gz = __fmul_rn(__fsub_rn(ra.z, I.lo[2]), I.inv[2]);
-          near = !(1.0f - (gx - floorf(gx)) > sn.x && 1.0f - (gy - floorf(gy)) > sn.y && 1.0f - (gz - floorf(gz)) > sn.z);
-        } else {
-          near = near_forward_face<kSingle>(p, k);
-        }
+      }
+      if (kHasBim && kSingle) {
+        near = near_forward_face(ra, lim, p.inst0.inv, p.near_shift);
+      } else if (kHasBim) {
+        const float4* grid = &p.near_grid[2u * (rec_w(ra) >> 16)];
+        const float4 a = __ldg(grid), b = __ldg(grid + 1);
+        const float inv[3] = {a.x, a.y, a.z}, shift[3] = {b.x, b.y, b.z};
+        near = near_forward_face(ra, lim, inv, shift);
       }
     }
     if (kHasBim) {
