@@ -288,9 +288,13 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_bin(const __grid_constant__
 // cost varies with the panels near the record (one sphere against a mesh
 // of many triangles), and the queue holds neighbouring records together,
 // so warps take 32 queue entries at a time from a counter until the queue
-// is empty: a warp of slow walks does not hold the others' share.
+// is empty: a warp of slow walks does not hold the others' share.  Bound by
+// the latency of its load chains.  c3 in a cell, 2M / 16M particles: 84 / 102
+// us before the finer panel grid and the panel heads in one load; then 39 /
+// 66 us at four CTAs per SM (64 registers, spills), 36 / 60 at three, 36 / 65
+// at two.
 template <bool kTable, bool kSingle>
-__global__ void __launch_bounds__(256, 4) k_bin_surface(KParams p) {
+__global__ void __launch_bounds__(256, 3) k_bin_surface(KParams p) {
   __shared__ DevSpecies s_species[kSingle ? kCtxSpecies : 1];
   __shared__ DevUni s_uni[kSingle ? kCtxUni : 1];
   SingleCtx ctx{};

@@ -46,6 +46,22 @@ __device__ __forceinline__ V3 axpy3(float t, const V3& b, const V3& a) {
 }
 __device__ __forceinline__ V3 ld3(const float* p) { return V3{p[0], p[1], p[2]}; }
 
+// What the side test, the normal and the reflection of a panel read: the
+// first half of its DevPanel, in three 16-byte loads.  The walk is a chain of
+// dependent loads; field by field, the shape had to arrive before the loads
+// it asks for began.
+struct PanelHead {
+  uint32_t shape, surface, axis;
+  float front, a[3], r, r2, n[3];
+};
+__device__ __forceinline__ PanelHead panel_head(const DevPanel* q) {
+  static_assert(sizeof(PanelHead) == 48 && sizeof(DevPanel) == 96, "three 16-byte loads, rows of 96 bytes");
+  PanelHead h;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) reinterpret_cast<uint4*>(&h)[k] = __ldg(reinterpret_cast<const uint4*>(q) + k);
+  return h;
+}
+
 // Component of w perpendicular to the unit axis n.
 __device__ __forceinline__ V3 perp3(const V3& w, const V3& n) {
   const float t = dot3(w, n);
@@ -53,7 +69,7 @@ __device__ __forceinline__ V3 perp3(const V3& w, const V3& n) {
 }
 
 // Signed side value of x for panel P: > 0 on the front face.
-__device__ __forceinline__ float panel_side(const DevPanel& P, const V3& x) {
+__device__ __forceinline__ float panel_side(const PanelHead& P, const V3& x) {
   const V3 a = ld3(P.a);
   float s;
   switch (P.shape) {
@@ -88,18 +104,18 @@ __device__ __forceinline__ float edge_test(const V3& e, const V3& w, const V3& n
 }
 
 // Does the crossing point c of a curved panel lie on the panel?
-__device__ __forceinline__ bool curved_on_panel(const DevPanel& P, const V3& c) {
+__device__ __forceinline__ bool curved_on_panel(const PanelHead& P, const DevPanel* Q, const V3& c) {
   if (P.shape == kPanelSph) return true;
   const float h = dot3(sub3(c, ld3(P.a)), ld3(P.n));
   if (P.shape == kPanelHemi) return h <= 0.0f;
-  return h >= 0.0f && h <= P.len;  // cylinder between its ends
+  return h >= 0.0f && h <= Q->len;  // cylinder between its ends
 }
 
 // First crossing of the segment x0 -> x1 (side values s0, s1) with P.
 // Returns true with the fraction t in [0, 1] and the face the segment
 // arrives from (true = front).
-__device__ __forceinline__ bool panel_cross(const DevPanel& P, const V3& x0, const V3& x1, float s0, float s1,
-                                            float& t, bool& face_front) {
+__device__ __forceinline__ bool panel_cross(const PanelHead& P, const DevPanel* Q, const V3& x0, const V3& x1, float s0,
+                                            float s1, float& t, bool& face_front) {
   const bool f0 = s0 > 0.0f, f1 = s1 > 0.0f;
   const V3 d = sub3(x1, x0);
   if (P.shape == kPanelRect || P.shape == kPanelTri || P.shape == kPanelDisk) {
@@ -110,14 +126,14 @@ __device__ __forceinline__ bool panel_cross(const DevPanel& P, const V3& x0, con
     if (P.shape == kPanelRect) {
       const uint32_t u = P.axis == 0 ? 1u : 0u, v = P.axis == 2 ? 1u : 2u;
       const float cu = comp(c, u), cv = comp(c, v);
-      return P.bounds[0] <= cu && cu <= P.bounds[1] && P.bounds[2] <= cv && cv <= P.bounds[3];
+      return Q->bounds[0] <= cu && cu <= Q->bounds[1] && Q->bounds[2] <= cv && cv <= Q->bounds[3];
     }
     const V3 a = ld3(P.a), n = ld3(P.n);
     if (P.shape == kPanelDisk) {
       const V3 w = sub3(c, a);
       return dot3(w, w) <= P.r2;
     }
-    const V3 b = ld3(P.v1), e = ld3(P.v2);
+    const V3 b = ld3(Q->v1), e = ld3(Q->v2);
     return edge_test(sub3(b, a), sub3(c, a), n) >= 0.0f && edge_test(sub3(e, b), sub3(c, b), n) >= 0.0f &&
            edge_test(sub3(a, e), sub3(c, e), n) >= 0.0f;
   }
@@ -148,17 +164,17 @@ __device__ __forceinline__ bool panel_cross(const DevPanel& P, const V3& x0, con
   if (in0) {  // leaving: the far root
     t = t2;
     face_front = f0;
-    return curved_on_panel(P, axpy3(t2, d, x0));
+    return curved_on_panel(P, Q, axpy3(t2, d, x0));
   }
   if (in1) {  // entering: the near root
     t = t1;
     face_front = f0;
-    return curved_on_panel(P, axpy3(t1, d, x0));
+    return curved_on_panel(P, Q, axpy3(t1, d, x0));
   }
   // both ends outside: through the object only if the near root is on the
   // segment; the far root (leaving) counts where the near one misses the panel
   if (!(raw1 >= 0.0f && raw1 <= 1.0f)) return false;
-  if (curved_on_panel(P, axpy3(t1, d, x0))) {
+  if (curved_on_panel(P, Q, axpy3(t1, d, x0))) {
     t = t1;
     face_front = f0;
     return true;
@@ -166,12 +182,12 @@ __device__ __forceinline__ bool panel_cross(const DevPanel& P, const V3& x0, con
   if (P.shape == kPanelSph) return false;
   t = t2;
   face_front = !f0;
-  return curved_on_panel(P, axpy3(t2, d, x0));
+  return curved_on_panel(P, Q, axpy3(t2, d, x0));
 }
 
 // Unit normal of P at the crossing point c, pointing to the front face; false
 // where it is undefined (c on a curved panel's axis or centre).
-__device__ __forceinline__ bool front_normal(const DevPanel& P, const V3& c, V3& m) {
+__device__ __forceinline__ bool front_normal(const PanelHead& P, const V3& c, V3& m) {
   switch (P.shape) {
     case kPanelRect:
       m = V3{P.axis == 0 ? P.front : 0.0f, P.axis == 1 ? P.front : 0.0f, P.axis == 2 ? P.front : 0.0f};
@@ -193,7 +209,7 @@ __device__ __forceinline__ bool front_normal(const DevPanel& P, const V3& c, V3&
 }
 
 // Mirror x1 in the tangent plane of P at c.
-__device__ __forceinline__ V3 panel_reflect(const DevPanel& P, const V3& c, const V3& x1) {
+__device__ __forceinline__ V3 panel_reflect(const PanelHead& P, const V3& c, const V3& x1) {
   if (P.shape == kPanelRect) {
     const float m = __fsub_rn(__fmul_rn(2.0f, comp(ld3(P.a), P.axis)), comp(x1, P.axis));
     return V3{P.axis == 0 ? m : x1.x, P.axis == 1 ? m : x1.y, P.axis == 2 ? m : x1.z};
@@ -207,7 +223,7 @@ __device__ __forceinline__ V3 panel_reflect(const DevPanel& P, const V3& c, cons
 // A point on face `want` (true = front) of P close to the crossing point c:
 // c itself, else c moved along the front normal by 2^-21 (|c|_1 + 1) times
 // 1, 4, 16, ... (8 tries).  Returns false when none of them is.
-__device__ __forceinline__ bool panel_nudge(const DevPanel& P, const V3& c, bool want, V3& q) {
+__device__ __forceinline__ bool panel_nudge(const PanelHead& P, const V3& c, bool want, V3& q) {
   q = c;
   if ((panel_side(P, c) > 0.0f) == want) return true;
   V3 m;
@@ -289,12 +305,12 @@ __device__ __forceinline__ bool surface_move(const SurfView& p, uint32_t sp, V3 
 #pragma unroll 1
           for (uint32_t k = __ldg(&p.start[box]); k < e; ++k) {
             const uint32_t id = __ldg(&p.list[k]);
-            const DevPanel& P = p.panels[id];
+            const PanelHead P = panel_head(&p.panels[id]);
             const uint8_t* act = &p.act[((size_t)P.surface * p.S + sp) * 2u];
             if (act[0] == kActTransmit && act[1] == kActTransmit) continue;  // invisible to sp
             float t;
             bool ff;
-            if (panel_cross(P, x0, x1, panel_side(P, x0), panel_side(P, x1), t, ff) &&
+            if (panel_cross(P, &p.panels[id], x0, x1, panel_side(P, x0), panel_side(P, x1), t, ff) &&
                 (t < best_t || (t == best_t && id < best))) {
               best_t = t;
               best = id;
@@ -303,7 +319,7 @@ __device__ __forceinline__ bool surface_move(const SurfView& p, uint32_t sp, V3 
           }
         }
     if (best == kNone) return true;
-    const DevPanel& P = p.panels[best];
+    const PanelHead P = panel_head(&p.panels[best]);
     const uint8_t action = p.act[((size_t)P.surface * p.S + sp) * 2u + (best_front ? 0u : 1u)];
     const V3 c = axpy3(best_t, sub3(x1, x0), x0);
     if (action == kActAbsorb) return false;
