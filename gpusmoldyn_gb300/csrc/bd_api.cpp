@@ -1475,6 +1475,7 @@ BD_API bd_status bd_synchronize(bd_handle h) {
       c.surf_ticket = 0;
       c.n_virtual = 0;
       c.bar_count = 0;
+      c.bar_word = 0;
       c.res_word = 0;
       c.res_left = 0;
       st = push_ctrl(h);

@@ -372,14 +372,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 // of two CTAs per SM (every CTA resident).  CTA b owns a contiguous range of
 // cells and moves it through shared memory in chunks of up to kScanChunk
 // counts, each brought in by one bulk copy (the copy engine, not a load
-// per word): pass 1 sums the range and publishes the sum (tile_sums[b]);
-// after one grid barrier, pass 2 adds the sums of the CTAs before it,
-// scans each chunk in shared memory (a contiguous run of counts per
-// thread) and writes it out by one bulk copy.  On the 16M c3 step a range
-// is one chunk, so pass 2 finds it still in shared memory.  The last 1..3
-// counts of the grid that do not fill 16 bytes go by plain loads and
-// stores.  20.8 us on the 16M c3 step; chunks of 49,152 counts (one CTA
-// per SM) took 22.4 us, of 12,288 (four) 26.3 us.  Earlier forms: a
+// per word): pass 1 sums the range, a contiguous run of counts per thread,
+// and publishes the sum (tile_sums[b]); after one grid barrier, pass 2 adds
+// the sums of the CTAs before it, scans each chunk in shared memory and
+// writes it out by one bulk copy.  On the 16M c3 step a range is one chunk,
+// so pass 2 finds it still in shared memory and its threads know where their
+// runs start.  The last 1..3 counts of the grid that do not fill 16 bytes go
+// by plain loads and stores.  What bounds it: its launch (6 us when it does
+// nothing) and the chain status, copy, barrier, sums, store.  c3 steps of 2M,
+// 4M, 14.5M and 16M particles: 9.9, 12.0, 17.9 and 18.0 us.  Runs of any
+// length, which meet in one bank when it is a multiple of 16, with a second
+// pass over the counts took 15.4, 19.8, 41.2 and 20.7 us.  At that time chunks
+// of 49,152 counts (one CTA per SM) took 22.4 us, of 12,288 (four) 26.3 us at
+// 16M.  Earlier forms: a
 // single-pass scan by decoupled look-back, 27 us (643 tiles, and the
 // frontier of known prefixes moved by the 32 flags one poll reads per round
 // trip); this grid scan reading tiles of 8,192 counts with vector loads
@@ -395,14 +400,16 @@ __device__ __forceinline__ void bulk_to_global(void* dst, const void* src, uint3
 }
 
 // Chunk [c0, c0 + len) of the counts into s_cnt: the 16-byte-aligned part
-// by one bulk copy (thread 0) on `bar`, the rest by plain loads.  False when
-// the copy's wait runs out.
-__device__ __forceinline__ bool scan_stage(const KParams& p, uint32_t* s_cnt, uint64_t* bar, uint32_t c0,
-                                           uint32_t len, uint32_t& phase) {
+// by one bulk copy on `bar` (scan_fetch, thread 0), the rest by plain loads.
+__device__ __forceinline__ void scan_fetch(const KParams& p, uint32_t* s_cnt, uint64_t* bar, uint32_t c0, uint32_t len) {
   const uint32_t bulk = len & ~3u;
-  if (bulk) {
-    if (threadIdx.x == 0) bulk_to_smem(s_cnt, p.cell_count + c0, bulk * 4u, bar);
-  }
+  if (bulk && threadIdx.x == 0) bulk_to_smem(s_cnt, p.cell_count + c0, bulk * 4u, bar);
+}
+
+// The fetched chunk is there.  False when the copy's wait runs out.
+__device__ __forceinline__ bool scan_landed(const KParams& p, uint32_t* s_cnt, uint64_t* bar, uint32_t c0, uint32_t len,
+                                            uint32_t& phase) {
+  const uint32_t bulk = len & ~3u;
   if (threadIdx.x < len - bulk) s_cnt[bulk + threadIdx.x] = __ldcg(&p.cell_count[c0 + bulk + threadIdx.x]);
   bool ok = true;
   if (bulk) {
@@ -417,57 +424,67 @@ __device__ __forceinline__ bool scan_stage(const KParams& p, uint32_t* s_cnt, ui
 __global__ void __launch_bounds__(1024) k_scan(KParams p) {
   extern __shared__ __align__(128) uint32_t s_cnt[];
   __shared__ __align__(8) uint64_t s_bar;
-  __shared__ uint32_t s_stop, s_total, s_prefix, s_warp[32];
+  __shared__ uint32_t s_stop, s_total, s_warp[32];
   DevCtrl* c = p.ctrl;
-  if (threadIdx.x == 0) {
-    s_stop = ld_u32(&c->status) != 0u;
-    mbar_init(&s_bar);
-    mbar_init_fence();
-  }
-  __syncthreads();
-  // the status is the previous kernels' and the same for every CTA: all
-  // return here together or none does
-  if (s_stop) return;
-  if (p.scan_withhold && blockIdx.x == 0) {  // test switch: CTA 0 never arrives
-    if (gridDim.x == 1 && threadIdx.x == 0) atomicOr(&c->status, kStatTimeout);
-    return;
-  }
   // ranges of a multiple of 4 counts (16-byte aligned bulk copies)
   const uint32_t per = ((p.n_cells + gridDim.x - 1u) / gridDim.x + 3u) & ~3u;
   const uint32_t lo = min(blockIdx.x * per, p.n_cells), hi = min(lo + per, p.n_cells);
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
   uint32_t phase = 0;
+  if (threadIdx.x == 0) {
+    const uint32_t status = ld_u32(&c->status);
+    mbar_init(&s_bar);
+    mbar_init_fence();
+    // the first chunk is on its way while the status is
+    if (lo < hi) scan_fetch(p, s_cnt, &s_bar, lo, min(kScanChunk, hi - lo));
+    s_stop = status != 0u;
+  }
+  __syncthreads();
+  // The status is the previous kernels' and the same for every CTA: all
+  // return here together or none does, once the copy has landed.
+  if (s_stop) {
+    if (lo < hi) scan_landed(p, s_cnt, &s_bar, lo, min(kScanChunk, hi - lo), phase);
+    return;
+  }
+  if (p.scan_withhold && blockIdx.x == 0) {  // test switch: CTA 0 never arrives
+    if (lo < hi) scan_landed(p, s_cnt, &s_bar, lo, min(kScanChunk, hi - lo), phase);
+    if (gridDim.x == 1 && threadIdx.x == 0) atomicOr(&c->status, kStatTimeout);
+    return;
+  }
   bool ok = true;
-  // pass 1: the range's sum
+  // A thread's run of a chunk is of odd length, so that a warp's runs start
+  // in different banks.
+  auto run_of = [](uint32_t len) { return ((len + 1023u) >> 10) | 1u; };
+  // pass 1: the range's sum, each thread over its run
   uint32_t sum = 0;
   for (uint32_t c0 = lo; c0 < hi && ok; c0 += kScanChunk) {
-    const uint32_t len = min(kScanChunk, hi - c0);
-    if (c0 != lo) __syncthreads();  // the previous chunk is summed
-    ok = scan_stage(p, s_cnt, &s_bar, c0, len, phase);
-    for (uint32_t i = threadIdx.x; i < len; i += 1024u) sum += s_cnt[i];
+    const uint32_t len = min(kScanChunk, hi - c0), q = run_of(len);
+    if (c0 != lo) {
+      __syncthreads();  // the previous chunk is summed
+      scan_fetch(p, s_cnt, &s_bar, c0, len);
+    }
+    ok = scan_landed(p, s_cnt, &s_bar, c0, len, phase);
+    const uint32_t b0 = min(threadIdx.x * q, len), b1 = min(b0 + q, len);
+    for (uint32_t i = b0; i < b1; ++i) sum += s_cnt[i];
   }
   if (!ok) {
     if (threadIdx.x == 0) atomicOr(&c->status, kStatTimeout);
     return;
   }
-  sum = __reduce_add_sync(kFull, sum);
-  if (lane == 0) s_warp[warp] = sum;
-  __syncthreads();
-  if (warp == 0) {
-    const uint32_t t = __reduce_add_sync(kFull, lane < (blockDim.x >> 5) ? s_warp[lane] : 0u);
-    if (lane == 0) p.tile_sums[blockIdx.x] = t;
-  }
+  // counts of the range before the thread's runs: its start in the chunk,
+  // when the range is one chunk
+  const uint32_t before = block_exclusive_scan<1024>(sum, &s_total);
+  if (threadIdx.x == 0) p.tile_sums[blockIdx.x] = s_total;
   if (!grid_barrier(c)) return;
-  // the counts before the range
-  if (warp == 0) {
-    uint32_t v = 0;
-    for (uint32_t b = lane; b < blockIdx.x; b += 32u) v += __ldcg(&p.tile_sums[b]);
-    v = __reduce_add_sync(kFull, v);
-    if (lane == 0) s_prefix = v;
-  }
+  // the counts before the range: all sums asked for at once, and every warp
+  // adds up the warps' sums for itself
+  uint32_t v = 0;
+  for (uint32_t b = threadIdx.x; b < blockIdx.x; b += 1024u) v += __ldcg(&p.tile_sums[b]);
+  v = __reduce_add_sync(kFull, v);
+  if (lane == 0) s_warp[warp] = v;
   __syncthreads();
-  // pass 2: each chunk scanned in shared memory, a run of q counts per thread
-  uint32_t carry = s_prefix;
+  uint32_t carry = __reduce_add_sync(kFull, s_warp[lane]);
+  // pass 2: each chunk's starts in shared memory, a run of q counts per thread
   const bool resident = hi - lo <= kScanChunk;  // the one chunk is still staged
   for (uint32_t c0 = lo; c0 < hi; c0 += kScanChunk) {
     const uint32_t len = min(kScanChunk, hi - c0);
@@ -475,17 +492,22 @@ __global__ void __launch_bounds__(1024) k_scan(KParams p) {
       __syncthreads();
       if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // last chunk's store has read its source
       __syncthreads();
-      if (!scan_stage(p, s_cnt, &s_bar, c0, len, phase)) {
+      scan_fetch(p, s_cnt, &s_bar, c0, len);
+      if (!scan_landed(p, s_cnt, &s_bar, c0, len, phase)) {
         if (threadIdx.x == 0) atomicOr(&c->status, kStatTimeout);
         break;
       }
     }
-    const uint32_t q = (len + 1023u) >> 10;
+    const uint32_t q = run_of(len);
     const uint32_t b0 = min(threadIdx.x * q, len), b1 = min(b0 + q, len);
-    uint32_t s = 0;
-    for (uint32_t i = b0; i < b1; ++i) s += s_cnt[i];
-    uint32_t run = carry + block_exclusive_scan<1024>(s, &s_total);
-    carry += s_total;
+    uint32_t run = carry + before, total = s_total;
+    if (!resident) {
+      uint32_t s = 0;
+      for (uint32_t i = b0; i < b1; ++i) s += s_cnt[i];
+      run = carry + block_exclusive_scan<1024>(s, &s_total);
+      total = s_total;
+    }
+    carry += total;
     for (uint32_t i = b0; i < b1; ++i) {
       const uint32_t x = s_cnt[i];
       s_cnt[i] = run;

