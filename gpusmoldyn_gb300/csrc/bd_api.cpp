@@ -32,10 +32,11 @@ using namespace bd;
 namespace {
 
 constexpr int kGraphBatch = 16;
-// Cells up to which a binned step runs in k_resident.  A c2 step takes, there
-// and as a chain of kernels (us): 1,000 particles 10.4 / 23.6, 100,000 23.5 /
-// 32.2, 1M (333,333 cells) 54.2 / 56.0, 1.2M 59.7 / 60.3, 2M 90.9 / 83.9.
-constexpr uint32_t kResidentCells = 400000;
+// Cells up to which a binned step runs in k_resident.  A c2 step (3 particles
+// a cell) takes, there and as a chain of kernels (us): 1,000 particles 10.2 /
+// 21.1, 100,000 22.9 / 27.0, 300,000 32.0 / 32.5, 600,000 40.6 / 40.1, 1M
+// 51.5 / 48.8, 1.2M 56.4 / 52.1.  c3 the same within 1.
+constexpr uint32_t kResidentCells = 150000;
 // Mean zeroth-order births per step that one CTA counts and bins beside the
 // others' records (k_resident, k_bin); more are counted by k_zeroth and dealt
 // out over the grid.

@@ -38,13 +38,14 @@ def system(n, cells, kon=0.5, births=0.0, seed=91, **kw):
     (3000, 7, 70, 35),
     (40000, 31, 6, 3),        # 29,791 cells: starts in shared memory
     (40000, 33, 6, 3),        # 35,937: a range per CTA
-    (200000, 73, 4, 2),       # 389,017: the most cells in one launch
-    (200000, 74, 4, 2),       # 405,224: the kernel chain
+    (200000, 53, 4, 2),       # 148,877: the most cells in one launch
+    (200000, 54, 4, 2),       # 157,464: the kernel chain
+    (200000, 74, 4, 2),       # 405,224
 ], ids=lambda v: str(v))
 def test_steps_in_one_launch_bit_exact(n, cells, steps, batch):
     s = system(n, cells, births=3.0 if n > 1 else 0.0)
     assert int(np.prod(s.grid()[0].astype(np.int64))) == cells ** 3
-    resident = cells < 74
+    resident = cells < 54
     assert s.kernels_per_step() == 1 if resident else s.kernels_per_step() > 1
     run_parity(s, steps, batch=batch)
     s.close()
