@@ -54,6 +54,36 @@ __device__ __forceinline__ U4 philox_keys(U4 c, const uint32_t (&keys)[kPhiloxKe
   return c;
 }
 
+// The same in two parts, for many blocks (i, t, tag, 0) of one i: what the
+// first three rounds compute from i and tag alone, and the block of a t.
+// Seven of the ten rounds and half of the third remain per t; the product of
+// the second round's x is the same for all i.
+struct PhiloxRow {
+  uint32_t z2, x3, z3, w3;  // of rounds 2 and 3, but for what depends on t
+};
+
+__device__ __forceinline__ PhiloxRow philox_row(uint32_t i, uint32_t tag, const uint32_t (&keys)[kPhiloxKeys]) {
+  const uint64_t p0 = (uint64_t)0xD2511F53u * i, p1 = (uint64_t)0xCD9E8D57u * tag;
+  const uint64_t q1 = (uint64_t)0xCD9E8D57u * ((uint32_t)(p0 >> 32) ^ keys[1]);
+  const uint64_t r0 = (uint64_t)0xD2511F53u * ((uint32_t)(q1 >> 32) ^ (uint32_t)p1 ^ keys[2]);
+  return PhiloxRow{(uint32_t)p0 ^ keys[3], (uint32_t)q1 ^ keys[4], (uint32_t)(r0 >> 32) ^ keys[5], (uint32_t)r0};
+}
+
+__device__ __forceinline__ U4 philox_of_row(const PhiloxRow& row, uint32_t t, uint32_t tag,
+                                            const uint32_t (&keys)[kPhiloxKeys]) {
+  const uint64_t q0 = (uint64_t)0xD2511F53u * ((uint32_t)(((uint64_t)0xCD9E8D57u * tag) >> 32) ^ t ^ keys[0]);
+  const uint64_t r1 = (uint64_t)0xCD9E8D57u * ((uint32_t)(q0 >> 32) ^ row.z2);
+  U4 c{(uint32_t)(r1 >> 32) ^ row.x3, (uint32_t)r1, (uint32_t)q0 ^ row.z3, row.w3};
+#pragma unroll
+  for (int r = 3; r < 10; ++r) {
+    const uint64_t p0 = (uint64_t)0xD2511F53u * c.x;
+    const uint64_t p1 = (uint64_t)0xCD9E8D57u * c.z;
+    c = U4{(uint32_t)(p1 >> 32) ^ c.y ^ keys[2 * r], (uint32_t)p1, (uint32_t)(p0 >> 32) ^ c.w ^ keys[2 * r + 1],
+           (uint32_t)p0};
+  }
+  return c;
+}
+
 // The reference's randReal: a 32-bit word scaled by 2^-32 in float
 // (rand_kernel.cuh:32-36).  May round to 1.0f, which no coin accepts.
 __device__ __forceinline__ float u32_to_unit(uint32_t v) {
@@ -69,6 +99,22 @@ __device__ __forceinline__ float u24_to_unit(uint32_t v) {
 __device__ __forceinline__ double u53_to_unit(uint32_t a, uint32_t b) {
   const uint64_t m = ((uint64_t)(a >> 5) << 26) | (uint64_t)(b >> 6);
   return (double)m * 1.1102230246251565e-16;
+}
+
+// log and 1 / sqrt of a normal number by the hardware's approximations.  The
+// bits are those of __logf and rsqrtf (compared for every 24-bit uniform and
+// the radii they give), without the instructions that scale a subnormal
+// argument, which a uniform of 2^-25 or more and a radius of 1e-30 or more
+// never are.
+__device__ __forceinline__ float log_normal(float x) {
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return 0.69314718055994531f * y;
+}
+__device__ __forceinline__ float rsqrt_normal(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 
 // Three standard normals from words x, y, z of one Philox block; word w is
@@ -90,10 +136,10 @@ __device__ __forceinline__ void normals3(const U4& r, const float* __restrict__ 
     // errors ~1e-6, far below the statistical resolution of the step
     const float a = u24_to_unit(r.x) + 2.98023223876953125e-08f;  // (0, 1)
     const float c = u24_to_unit(r.z) + 2.98023223876953125e-08f;
-    // __logf may round to 0 just below 1: keep the radius finite (0)
-    const float la = fmaxf(-2.0f * __logf(a), 1e-30f), lc = fmaxf(-2.0f * __logf(c), 1e-30f);
-    const float ra = la * rsqrtf(la);
-    const float rc = lc * rsqrtf(lc);
+    // the log may round to 0 just below 1: keep the radius finite (0)
+    const float la = fmaxf(-2.0f * log_normal(a), 1e-30f), lc = fmaxf(-2.0f * log_normal(c), 1e-30f);
+    const float ra = la * rsqrt_normal(la);
+    const float rc = lc * rsqrt_normal(lc);
     float sa, ca, sc, cc;
     __sincosf(6.2831853071795865f * u24_to_unit(r.y), &sa, &ca);
     const uint32_t low = ((r.x & 0xFFu) << 24) | ((r.y & 0xFFu) << 16) | ((r.z & 0xFFu) << 8);

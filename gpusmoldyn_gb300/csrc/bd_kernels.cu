@@ -585,13 +585,17 @@ __global__ void __launch_bounds__(1024) k_match(KParams p) {
 // Nothing in a diffusion-only step depends on another record, so a record
 // takes all its steps in registers: one read and one write whatever their
 // number, one launch, and no k_finalize_inplace (the last CTA to finish
-// commits).  Bound by the issue of Philox and Box-Muller: 16 steps of 1M
-// records, with the caller's call, wait and copy of the records, took 297 us
-// as 32 launches and take 155 us; the memory floor is 5 us.  Same operations
-// in the same order as advance_rec, so the same bits.  Without zeroth-order
-// reactions; with them the slot count changes every step.
+// commits).  Bound by the issue of Philox and Box-Muller, 3.7 us a step of 1M
+// records (4.3 before the rows of philox_row, two steps unrolled, one in-box
+// test and the subnormal cases left out of the normals), beside a memory floor
+// of 5 us in all: 16 steps took 224 us as 32 launches, 80 with those, 76 now.
+// Same operations in the same order as advance_rec, so the same bits.
+// Without zeroth-order reactions; with them the slot count changes every
+// step.
+constexpr uint32_t kDiffuseCtas = 8;  // per SM
+
 template <bool kTable>
-__global__ void __launch_bounds__(256) k_diffuse_steps(KParams p, uint32_t nsteps) {
+__global__ void __launch_bounds__(256, (int)kDiffuseCtas) k_diffuse_steps(const __grid_constant__ KParams p, uint32_t nsteps) {
   DevCtrl* c = p.ctrl;
   if (ctrl_status_warp(c)) return;
   const uint32_t n = ld_u32(&c->n_slots), cur = ld_u32(&c->cur);
@@ -601,18 +605,31 @@ __global__ void __launch_bounds__(256) k_diffuse_steps(KParams p, uint32_t nstep
   const uint32_t take = advancing(flags) ? min(nsteps, max(target, step0 + 1u) - step0) : 0u;
   float4* st = cur ? p.state[1] : p.state[0];
   const DevInstance& I = p.inst0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  // 32 records at a time, dealt to the CTAs in turn: what is left for a last
+  // round is spread over the SMs
+  const uint32_t first = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32u + lane_id();
+  for (uint64_t at = first; at < n; at += gridDim.x * blockDim.x) {
+    const uint32_t i = (uint32_t)at;
     float4 r = st[i];
     const uint32_t w = rec_w(r);
     if (w == kDead || take == 0) continue;
     const float sigma = __ldg(&p.species[I.block * p.S + (w & kSpeciesMask)].sigma);
+    const PhiloxRow row = philox_row(i - base, kTagDiffuse, p.keys0);
+#pragma unroll 2
     for (uint32_t k = 0; k < take; ++k) {
-      const U4 rn = philox(U4{i - base, step0 + k, kTagDiffuse, 0u}, I.key_lo, I.key_hi);
+      const U4 rn = philox_of_row(row, step0 + k, kTagDiffuse, p.keys0);
       float g0, g1, g2;
       normals3<kTable>(rn, p.gauss, g0, g1, g2);
-      r.x = reflect(__fmaf_rn(sigma, g0, r.x), I.lo[0], I.hi[0]);
-      r.y = reflect(__fmaf_rn(sigma, g1, r.y), I.lo[1], I.hi[1]);
-      r.z = reflect(__fmaf_rn(sigma, g2, r.z), I.lo[2], I.hi[2]);
+      r.x = __fmaf_rn(sigma, g0, r.x);
+      r.y = __fmaf_rn(sigma, g1, r.y);
+      r.z = __fmaf_rn(sigma, g2, r.z);
+      // one branch for the three axes
+      if (!(r.x >= I.lo[0] && r.x <= I.hi[0] && r.y >= I.lo[1] && r.y <= I.hi[1] && r.z >= I.lo[2] &&
+            r.z <= I.hi[2])) {
+        r.x = reflect(r.x, I.lo[0], I.hi[0]);
+        r.y = reflect(r.y, I.lo[1], I.hi[1]);
+        r.z = reflect(r.z, I.lo[2], I.hi[2]);
+      }
     }
     st[i] = r;
   }
@@ -837,9 +854,14 @@ void launch_scan(const KParams& p, const LaunchShape& shape, cudaStream_t s) {
 }
 
 void enqueue_diffuse(const KParams& p, bool table, uint32_t nsteps, uint64_t n_slots, cudaStream_t s) {
-  // a record per thread: the work of a record is long and the same for all
-  const uint64_t ctas = (n_slots + 255u) / 256u;
-  const unsigned grid = (unsigned)std::min<uint64_t>(std::max<uint64_t>(ctas, 1u), 1u << 20);
+  // Few steps: one wave, since a CTA's reads of the control words, its fence
+  // and its count take longer than a record's step.  Many: a CTA per 256
+  // records, since the last round of a wave runs half empty.  One wave and a
+  // CTA per 256 records, us: 1M records 1 step 17 / 51, 8 steps 43 / 59, 16
+  // steps 75 / 77, 25 steps 111 / 107; 4M 34 / 182, 140 / 204, 262 / 271,
+  // 406 / 384.
+  const uint64_t ctas = std::max<uint64_t>((n_slots + 255u) / 256u, 1u);
+  const unsigned grid = (unsigned)std::min<uint64_t>(ctas, nsteps < 20u ? 152u * kDiffuseCtas : 1u << 20);
   if (table) k_diffuse_steps<true><<<grid, 256, 0, s>>>(p, nsteps);
   else k_diffuse_steps<false><<<grid, 256, 0, s>>>(p, nsteps);
 }

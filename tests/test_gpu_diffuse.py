@@ -26,6 +26,8 @@ def system(n, D=(1.0, 0.1, 0.0), side=2.0):
     (1, 130, 130, (1.0,)),            # three launches
     (257, 66, 33, (1.0, 0.1, 0.0)),
     (100003, 6, 3, (1.0, 0.1, 0.0)),
+    (400003, 4, 3, (1.0, 0.1, 0.0)),  # more than a wave of records, few steps
+    (400003, 21, 21, (1.0,)),         # and many
     (1000, 4, 2, (5000.0, 1.0)),      # steps that cross the box several times
 ])
 def test_diffusion_steps_in_one_launch_bit_exact(n, steps, batch, D):
