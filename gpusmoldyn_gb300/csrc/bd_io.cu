@@ -128,6 +128,15 @@ __global__ void __launch_bounds__(kIoThreads) k_export_write(ExportArgs a) {
   }
 }
 
+__global__ void __launch_bounds__(256) k_export_all(ExportArgs a) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n_slots; i += stride) {
+    const float4 r = a.state[i];
+    a.xyz4[i] = make_float4(r.x, r.y, r.z, 1.0f);
+    a.species[i] = (int)(__float_as_uint(r.w) & 0xFFFFu);
+  }
+}
+
 int grid_for(uint64_t n) {
   const uint64_t g = (n + 255) / 256;
   return (int)(g < 1 ? 1 : (g > 152 * 16 ? 152 * 16 : g));
@@ -153,6 +162,10 @@ void enqueue_export(const ExportArgs& a, cudaStream_t s) {
   k_export_count<<<a.n_tiles, kIoThreads, 0, s>>>(a);
   k_export_scan<<<1, kIoThreads, 0, s>>>(a);
   k_export_write<<<a.n_tiles, kIoThreads, 0, s>>>(a);
+}
+
+void enqueue_export_all(const ExportArgs& a, cudaStream_t s) {
+  if (a.n_slots) k_export_all<<<grid_for(a.n_slots), 256, 0, s>>>(a);
 }
 
 }  // namespace bd

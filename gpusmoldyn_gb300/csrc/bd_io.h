@@ -39,5 +39,8 @@ struct ExportArgs {
 };
 uint32_t export_tiles(uint64_t n_slots);
 void enqueue_export(const ExportArgs& a, cudaStream_t s);
+// The same when every slot is exported (all instances, no empty slot): no
+// scratch, no count.
+void enqueue_export_all(const ExportArgs& a, cudaStream_t s);
 
 }  // namespace bd
