@@ -1,38 +1,47 @@
 // bd_kernels.cu -- the per-timestep kernels of the Brownian-dynamics step.
 //
-// Sorted path (any first- or second-order reaction, or an ensemble), one
-// step = 7 or 8 launches, no host synchronisation, all counts on the device:
+// A step of a reacting system is a chain of kernels with no host
+// synchronisation, all counts on the device; their phases are the functions of
+// bd_step.cuh, which bd_resident.cu runs in one kernel for small systems.
 //
-//   k_zeroth    1 CTA      Poisson birth counts of the zeroth-order reactions
-//                          (zeroReact + poisrandF on the host in the
-//                          reference, reaction_cpu.cpp:36-63, stats.cpp:234-275)
-//   k_count     streaming  diffuse + reflect + first-order reactions + cell key,
-//                          warp-aggregated cell histogram; writes nothing else
-//                          (diffuse, uniReact, adjustPositions, calcHashD:
-//                          particles_kernel.cu:61-95, 127-207,
-//                          reaction_kernel.cuh:263-342)
-//   k_scan_*    3 launches exclusive scan of the cell histogram = cell starts
-//                          (replaces RadixSort's 5 passes + CUDPP scans,
-//                          radixsort.cu:1045-1143, and the cellStart memset)
-//   k_scatter   streaming  recomputes k_count's records (counter-based RNG makes
-//                          them identical) and scatters each into its cell;
-//                          dead particles get no slot, births get one
-//                          (compactPosAndTypeD, particles_kernel.cu:98-123)
-//   k_pairs     streaming  canonical order inside each cell + pair search over
-//                          the neighbour cells within the binding radius
-//                          (reorderDataAndFindCellStartD, collideD, collideCell:
-//                          particles_kernel.cu:212-272, 318-497)
-//   k_match     1 CTA      one reaction per particle (greedy matching in pair
-//                          order), product placement, counters, commit
-//                          (bimReact, resetNonInteracting: reaction_kernel.cuh:
-//                          202-258, particles_kernel.cu:499-508)
+// Binned sort (the default), 5 launches, 6 with surface panels:
+//   k_bin          streaming  diffuse + reflect + first-order reactions + cell
+//                             key, each record into the next place of its
+//                             cell's bin; births last (diffuse, uniReact,
+//                             adjustPositions, calcHashD: particles_kernel.cu:
+//                             61-95, 127-207, reaction_kernel.cuh:263-342;
+//                             zeroReact + poisrandF on the host in the
+//                             reference, reaction_cpu.cpp:36-63, stats.cpp:
+//                             234-275)
+//   k_bin_surface  streaming  the records whose move meets a panel
+//   k_scan         one wave   exclusive scan of the cell counts = cell starts
+//                             (replaces RadixSort's 5 passes + CUDPP scans,
+//                             radixsort.cu:1045-1143, and the cellStart memset)
+//   k_pairs_cells  streaming  canonical order inside each cell + pair search
+//                             over the neighbour cells within the binding
+//                             radius (reorderDataAndFindCellStartD, collideD,
+//                             collideCell: particles_kernel.cu:212-272,
+//                             318-497)
+//   k_pairs_big    one wave   the same for cells of more than kBigCell records
+//   k_match        32 CTAs    one reaction per particle (greedy matching in
+//                             pair order), product placement, counters, commit
+//                             (bimReact, resetNonInteracting:
+//                             reaction_kernel.cuh:202-258,
+//                             particles_kernel.cu:499-508)
+// More births than kFewBirths a step are counted by k_zeroth before it.
 //
-// HBM traffic per particle-step: k_count R16, k_scatter R16 + W16, k_pairs
-// R16 + W16 = 80 B, plus 4-12 B per cell for the histogram and the starts.
+// Compact sort (when the bins would not fit), 6 launches: k_count and
+// k_scatter in place of k_bin; k_scatter recomputes k_count's records
+// (counter-based RNG makes them identical) and puts each into its cell's range
+// (compactPosAndTypeD, particles_kernel.cu:98-123).
 //
-// Diffusion-only path (no first- or second-order reaction, one instance):
-// k_diffuse updates the records in place (R16 + W16) and zeroth-order births
-// are appended by k_append.
+// HBM traffic per particle-step: k_bin R16 + W16, k_pairs R16 + W16 = 64 B,
+// plus 12 B per cell for the counts and the starts; compact 16 B more.
+//
+// Diffusion alone (no first- or second-order reaction, one instance):
+// k_diffuse_steps takes many steps of each record in one launch; with
+// zeroth-order births k_diffuse updates the records in place and k_append
+// adds the births.
 #include "bd_step.cuh"
 
 namespace bd {

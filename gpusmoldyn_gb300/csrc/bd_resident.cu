@@ -1,14 +1,14 @@
 // bd_resident.cu -- several timesteps of a small binned system in one launch.
 //
-// One step as a chain of kernels (k_zeroth, k_bin, k_scan, k_pairs_cells,
-// k_pairs_big, k_match) costs 24 to 30 us however small the system: launches,
-// their ramps and the chains of dependent loads at the head of each kernel,
-// not the work.  (c2 steps, chain before and k_resident: 4,001 particles 31.4
-// -> 10.8 us, 40,000 34.7 -> 19, 300,007 of c3 44.5 -> 33, 1M 59.3 -> 54.6.)  Here the whole step runs
-// in one cooperative kernel that stays resident for many steps, and what
-// bounds it is round trips to L2 (0.4 us each): a barrier of the grid is
-// three of them.  So a step has as few barriers as it can: two when it has
-// no candidate pairs.
+// One step as a chain of kernels (k_bin, k_scan, k_pairs_cells, k_pairs_big,
+// k_match) costs 21 us however small the system: launches, their ramps and the
+// chains of dependent loads at the head of each kernel, not the work.  Here
+// the whole step runs in one cooperative kernel that stays resident for many
+// steps, and what bounds it is round trips to L2 (0.4 us each): a barrier of
+// the grid is three of them.  c2 steps, chain and here, us: 1,000 particles
+// 21.1 / 10.2, 40,000 25.8 / 16.5, 100,000 27.0 / 22.9, 300,000 32.5 / 32.0;
+// above that the chain is faster.  So a step has as few barriers as it can:
+// two when it has no candidate pairs.
 //   * The cell scan is not a phase: after binning every CTA scans all counts
 //     for itself into shared memory (up to kSmallCells cells; above that the
 //     CTAs scan a range each, at the price of two more barriers).
