@@ -276,10 +276,16 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_bin(const __grid_constant__
   __shared__ DevUni s_uni[kSingle ? kCtxUni : 1];
   __shared__ DeferBuffer s_defer[kSurf == 2 ? 8 : 1];  // one per warp (blocks of at most 256 threads)
   DeferBuffer& defer_buf = s_defer[kSurf == 2 ? threadIdx.x >> 5 : 0];
+  // One answer for the whole CTA: records binned by the other CTAs may raise
+  // a status bit at any time, and zeroth_births has barriers and a scan that
+  // every warp takes part in.
+  __shared__ uint32_t s_stop;
+  DevCtrl* c = p.ctrl;
+  if (threadIdx.x == 0) s_stop = ld_u32(&c->status);
   SingleCtx ctx{};
   if (kSingle) ctx = single_ctx(p, s_species, s_uni);
-  DevCtrl* c = p.ctrl;
-  if (ctrl_status_warp(c)) return;
+  else __syncthreads();
+  if (s_stop) return;
   const uint32_t cur = ld_u32(&c->cur);
   const float4* __restrict__ st = cur_state(p, cur);
   const uint32_t n_real = ld_u32(&c->n_slots);
