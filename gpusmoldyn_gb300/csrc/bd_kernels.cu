@@ -44,6 +44,8 @@
 // adds the births.
 #include "bd_step.cuh"
 
+#include <algorithm>
+
 namespace bd {
 namespace {
 
@@ -555,8 +557,9 @@ __global__ void __launch_bounds__(256, 4) k_pairs_cells(KParams p) {
 }
 
 // Large cells: part 1 (sort) by every CTA, a grid barrier, part 2 (pairs)
-// by every CTA, in one launch (cooperative when there are pairs to find,
-// so that the barrier waits only on resident CTAs).  Every CTA reads the
+// by every CTA, in one launch, cooperative whether there are pairs to find
+// or not (the merge passes of the sort have barriers too), so that a
+// barrier waits only on resident CTAs.  Every CTA reads the
 // same final count of queued cells, so when none is large they all leave
 // at once: one empty launch per step instead of two (the two empty
 // launches cost 3.3 us per 16M c3 step; the one measured within noise of
@@ -829,8 +832,8 @@ void launch_match(const KParams& p, const LaunchShape& shape, cudaStream_t s) {
   else cudaLaunchKernelEx(&cfg, k_match<false>, p);
 }
 
-// The large-cell kernel over shape.grid_big CTAs, cooperatively when it
-// has pairs to find (its grid barrier waits only on resident CTAs).
+// The large-cell kernel over shape.grid_big CTAs, cooperatively (its grid
+// barriers wait only on resident CTAs).
 void launch_big(const KParams& p, bool has_bim, bool binned, const LaunchShape& shape, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)std::max(shape.grid_big, 1));
@@ -841,7 +844,7 @@ void launch_big(const KParams& p, bool has_bim, bool binned, const LaunchShape& 
   attr.id = cudaLaunchAttributeCooperative;
   attr.val.cooperative = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = has_bim && shape.grid_big > 1 ? 1 : 0;
+  cfg.numAttrs = shape.grid_big > 1 ? 1 : 0;
   if (has_bim) {
     if (binned) cudaLaunchKernelEx(&cfg, k_pairs_big<true, true>, p);
     else cudaLaunchKernelEx(&cfg, k_pairs_big<true, false>, p);
@@ -1017,11 +1020,13 @@ int match_grid(int n_sm) {
 }
 
 int big_grid(int n_sm) {
-  int a = 0, b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_pairs_big<true, true>, 256, 0) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pairs_big<true, false>, 256, 0) != cudaSuccess)
+  int a[4] = {0, 0, 0, 0};
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a[0], k_pairs_big<true, true>, 256, 0) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a[1], k_pairs_big<true, false>, 256, 0) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a[2], k_pairs_big<false, true>, 256, 0) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a[3], k_pairs_big<false, false>, 256, 0) != cudaSuccess)
     return 1;
-  const int resident = (a < b ? a : b) * n_sm;
+  const int resident = *std::min_element(a, a + 4) * n_sm;
   return resident < 1 ? 1 : (resident < kBigGrid ? resident : kBigGrid);
 }
 

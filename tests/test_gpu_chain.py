@@ -1,11 +1,13 @@
 """The kernel chain of the binned sort (k_bin, k_scan, k_pairs_cells,
-k_pairs_big, k_match) on grids of more cells than k_resident takes, GPU
-against the oracle bit for bit.  Bits are compared, so there is no
+k_pairs_big, k_match), on grids of more cells than k_resident takes or with
+a panel, GPU against the oracle bit for bit.  Bits are compared, so there is no
 tolerance."""
 import numpy as np
 import pytest
 
+from gpusmoldyn_gb300 import _lib as L
 from gpusmoldyn_gb300.configs import rng, uniform_positions
+from gpusmoldyn_gb300.system import System
 from test_gpu_parity import run_parity
 from test_gpu_resident import system
 
@@ -25,4 +27,27 @@ def test_bins_overflow_beside_births_in_the_last_cta(births):
     s.set_particles(pos, (np.arange(3000) % 3).astype(np.int32))
     assert s.kernels_per_step() == 5  # no k_zeroth: the births are k_bin's
     run_parity(s, 6, batch=3)
+    s.close()
+
+
+@pytest.mark.parametrize("sort", ["binned", "compact"])
+@pytest.mark.parametrize("n", [2048, 2049, 4097, 65537])
+def test_large_cells_without_second_order_reactions(n, sort):
+    """Cells cut into units (2,048 records) and joined by one merge pass, or
+    by two above 32 units, in a network that has no pairs to find."""
+    s = System((-0.75,) * 3, (1.25,) * 3, dt=1e-3, seed=83, normals="table", sort=sort, cell_size=0.5)
+    A, B = s.add_species(0.2), s.add_species(0.1)
+    s.add_reaction(1, [A], [B], 30.0)
+    s.add_reaction(1, [B], [A, A], 20.0)
+    if sort == "binned":  # a panel nothing meets, so that the steps are the chain's
+        f = s.add_surface()
+        s.set_surface_action(f, L.BD_ALL_SPECIES, "both", "transmit")
+        s.add_panel(f, "rect", [1.2, -0.75, -0.75, 2.0, 2.0], axis=0)
+    s.finalize()
+    g = rng(83)
+    pos = np.concatenate([uniform_positions(g, n, (-0.15,) * 3, (0.15,) * 3),
+                          uniform_positions(g, 300, (0.4,) * 3, (1.25,) * 3)])
+    s.set_particles(pos, g.integers(0, 2, len(pos)).astype(np.int32))
+    assert s.kernels_per_step() > 1
+    run_parity(s, 2)
     s.close()
