@@ -286,7 +286,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident(const __grid_constant_
       }
     } else {
       // CTA 0 matches and commits while the others wait, unless so many
-      // candidates came up that every CTA has to take part
+      // candidates came up that every CTA has to take part.  The step's first-
+      // and zeroth-order events count with the commit, before the barrier that
+      // may report another CTA's failure in the next step: a committed step is
+      // not taken again.
+      auto count_events = [&]() {
+        if (kSingle && threadIdx.x < p.R && s_events[threadIdx.x])
+          p.events[threadIdx.x] = __ldcg(&p.events[threadIdx.x]) + s_events[threadIdx.x];
+      };
       uint32_t K = 0;
       if (blockIdx.x == 0) {
         K = ld_u32(&c->n_pairs);
@@ -297,17 +304,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_resident(const __grid_constant_
           flag_phase(kFlagGrid);
         } else {
           match_step(s_params, c, K, mine, false, s_match);
+          count_events();
         }
       }
       met = phase_barrier(c, bar, kGridReport);
       if (met & kMetFailure) break;
       if (met & kMetGrid) {
         if (!match_step(s_params, c, ld_u32(&c->n_pairs), DevPair{}, true, s_match)) return;
+        if (blockIdx.x == 0) count_events();
         if (phase_barrier(c, bar, kNothing) & kMetFailure) break;
       }
-      // the matching's events are in; now the rest of the step's
-      if (kSingle && blockIdx.x == 0 && threadIdx.x < p.R && s_events[threadIdx.x])
-        p.events[threadIdx.x] = __ldcg(&p.events[threadIdx.x]) + s_events[threadIdx.x];
     }
     // the next step's state
     cur ^= 1u;
