@@ -144,7 +144,7 @@ enum PanelShape : uint32_t { kPanelRect = 0, kPanelTri = 1, kPanelSph = 2, kPane
 enum SurfaceAction : uint8_t { kActTransmit = 0, kActReflect = 1, kActAbsorb = 2 };
 constexpr int kMaxSurfaceHits = 8;  // crossings handled per segment and step
 
-struct DevPanel {          // 96 B
+struct alignas(16) DevPanel {  // 96 B; its first half is read in three 16-byte loads
   uint32_t shape;          // PanelShape
   uint32_t surface;        // owning surface (index of its action table)
   uint32_t axis;           // rect: axis perpendicular to the panel

@@ -24,6 +24,8 @@
 //                    clamped to [0, 1]
 // A point exactly on a panel is on its back face.
 #pragma once
+#include <stddef.h>
+
 #include "bd_device.cuh"
 #include "bd_kernels.h"
 
@@ -55,11 +57,21 @@ struct PanelHead {
   float front, a[3], r, r2, n[3];
 };
 __device__ __forceinline__ PanelHead panel_head(const DevPanel* q) {
-  static_assert(sizeof(PanelHead) == 48 && sizeof(DevPanel) == 96, "three 16-byte loads, rows of 96 bytes");
-  PanelHead h;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) reinterpret_cast<uint4*>(&h)[k] = __ldg(reinterpret_cast<const uint4*>(q) + k);
-  return h;
+  static_assert(alignof(DevPanel) == 16 && sizeof(DevPanel) == 96, "16-byte loads, rows of 96 bytes");
+  static_assert(offsetof(DevPanel, shape) == 0 && offsetof(DevPanel, surface) == 4 && offsetof(DevPanel, axis) == 8 &&
+                    offsetof(DevPanel, front) == 12 && offsetof(DevPanel, a) == 16 && offsetof(DevPanel, r) == 28 &&
+                    offsetof(DevPanel, r2) == 32 && offsetof(DevPanel, n) == 36 && offsetof(DevPanel, len) == 48,
+                "the words taken apart below");
+  const uint4* w = reinterpret_cast<const uint4*>(q);
+  const uint4 u = __ldg(w), v = __ldg(w + 1), x = __ldg(w + 2);
+  return PanelHead{u.x,
+                   u.y,
+                   u.z,
+                   __uint_as_float(u.w),
+                   {__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z)},
+                   __uint_as_float(v.w),
+                   __uint_as_float(x.x),
+                   {__uint_as_float(x.y), __uint_as_float(x.z), __uint_as_float(x.w)}};
 }
 
 // Component of w perpendicular to the unit axis n.
