@@ -951,7 +951,14 @@ void plan_panel_grid(bd_system* h) {
       lo[k] = std::min(lo[k], d.box_lo[k]);
       hi[k] = std::max(hi[k], d.box_hi[k]);
     }
-  build_panel_grid(h->panels, lo, hi, &h->pgrid);
+  double step = 0.0;  // of the species that some panel stops
+  for (int sp = 0; sp < (int)h->D.size(); sp++) {
+    bool seen = false;
+    for (int f = 0; f < (int)h->surfaces.size(); f++)
+      seen |= surface_action(h, f, sp, 0) != kActTransmit || surface_action(h, f, sp, 1) != kActTransmit;
+    for (const DerivedParams& P : h->derived) step = seen ? std::max(step, (double)P.sigma[sp]) : step;
+  }
+  build_panel_grid(h->panels, lo, hi, step, &h->pgrid);
   // a step of species s walks s and the products of its first-order
   // reactions: the panel counts for s when any of them sees it
   const int S = (int)h->D.size();

@@ -198,21 +198,32 @@ bool panel_meets_box(const bd_panel_info& P, const double lo[3], const double hi
 
 }  // namespace
 
-void build_panel_grid(const std::vector<bd_panel_info>& panels, const float lo[3], const float hi[3], PanelGrid* g) {
+void build_panel_grid(const std::vector<bd_panel_info>& panels, const float lo[3], const float hi[3], double step,
+                      PanelGrid* g) {
   double ext[3], emax = 0.0;
   for (int k = 0; k < 3; k++) {
     ext[k] = std::max((double)hi[k] - lo[k], 1e-30);
     emax = std::max(emax, ext[k]);
   }
-  // About 512 boxes per panel, at most 64 per axis: a walk tests the panels of
-  // every box its segment touches, one after the other, so few panels per box
-  // matter more than few boxes.  1,281 panels (c3 in a cell, 2M particles):
-  // k_bin_surface 84 us with 8 boxes per panel, 53 with 64, 45 with 512; 41
-  // with 4,096 (128 per axis), where the tables take longer to build.
-  const double per_axis = std::ceil(std::cbrt(512.0 * (double)std::max<size_t>(panels.size(), 1)));
+  // At least 8 boxes per panel, up to 32 per axis; up to 512 per panel and 64
+  // per axis while a box is at least four rms steps wide.  A walk tests the
+  // panels of every box that its segment's bounding box touches, one after the
+  // other: few panels per box matter more than few boxes as long as a step
+  // touches few boxes (1,281 panels, c3 in a cell, 2M particles, k_bin_surface:
+  // 84 us with 8 boxes per panel, 53 with 64, 45 with 512; 41 with 4,096, where
+  // the tables take longer to build), and cost a test per box when it touches
+  // many.  200,000 particles, us a step with 8 boxes per panel / 512 / this
+  // rule: one rectangle, rms step 0.3 of the box 74 / 184 / 60; 80 triangles,
+  // step 0.03 102 / 114 / 83, 0.3 778 / 5,397 / 700; 1,280 triangles, step
+  // 0.003 85 / 62 / 62, 0.03 204 / 291 / 164, 0.1 970 / 2,940 / 815.  A box of
+  // two, six or eight steps is worse by up to 20% for some of these.
+  const double n_panels = (double)std::max<size_t>(panels.size(), 1);
+  const double coarse = std::ceil(std::cbrt(8.0 * n_panels)), fine = std::ceil(std::cbrt(512.0 * n_panels));
   for (int k = 0; k < 3; k++) {
-    const double n = std::ceil(per_axis * ext[k] / emax);
-    g->dims[k] = (uint32_t)std::min(64.0, std::max(1.0, n));
+    const double n = std::min(64.0, std::ceil(fine * ext[k] / emax));
+    const double least = std::min(32.0, std::max(1.0, std::ceil(coarse * ext[k] / emax)));
+    const double most = step > 0.0 ? std::floor(ext[k] / (4.0 * step)) : n;
+    g->dims[k] = (uint32_t)std::max(least, std::min(n, most));
     g->lo[k] = lo[k];
     g->inv[k] = (float)(g->dims[k] / ext[k]);
   }

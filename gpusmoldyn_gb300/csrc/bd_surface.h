@@ -16,7 +16,7 @@ namespace bd {
 // a message for a malformed panel.
 bd_status derive_panel(const bd_panel& in, int surface, bd_panel_info* out, std::string* msg);
 
-// Panel lists over a grid of at most 32 boxes per axis spanning [lo, hi]
+// Panel lists over a grid of at most 64 boxes per axis spanning [lo, hi]
 // (the edge boxes extend to infinity): every panel is listed in each box,
 // grown by 1e-3 of a box edge, that its bounding box touches and that the
 // panel itself can pass through (spheres and hemispheres by their surface,
@@ -29,7 +29,10 @@ struct PanelGrid {
   std::vector<uint32_t> start;  // [n_boxes + 1]
   std::vector<uint32_t> list;
 };
-void build_panel_grid(const std::vector<bd_panel_info>& panels, const float lo[3], const float hi[3], PanelGrid* g);
+// step: the rms step per axis of the fastest species that sees a panel; it
+// decides how fine the grid is, not what is listed.
+void build_panel_grid(const std::vector<bd_panel_info>& panels, const float lo[3], const float hi[3], double step,
+                      PanelGrid* g);
 
 // Species bit of the per-cell masks: species s < 7 has bit s, every species
 // from 7 on shares bit 7.
