@@ -565,8 +565,13 @@ __global__ void __launch_bounds__(256, 4) k_pairs_cells(KParams p) {
 // launches cost 3.3 us per 16M c3 step; the one measured within noise of
 // them).  The first step that queues a cell without big_scratch in place
 // raises kStatScratch; the host allocates it and replays the step.
+// 64 registers: at the 114 the compiler asks for, the two CTAs per SM hold
+// nearly every register, so that the launch, which needs all of them resident
+// at once, waits for the other handles' kernels to drain (8 handles of 40,000
+// particles, us a step of each: 70 with 114 registers, 50 with 64, 57 before
+// the units; 16 handles 142 / 99 / 113).  Its own time rises by 1 to 5%.
 template <bool kHasBim, bool kBinned>
-__global__ void __launch_bounds__(256) k_pairs_big(KParams p) {
+__global__ void __launch_bounds__(256, 4) k_pairs_big(KParams p) {
   __shared__ unsigned long long s_key[kBigChunk];
   DevCtrl* c = p.ctrl;
   if (stop_block(c)) return;
