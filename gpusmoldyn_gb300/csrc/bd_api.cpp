@@ -32,10 +32,8 @@ using namespace bd;
 namespace {
 
 constexpr int kGraphBatch = 16;
-// Cells up to which a binned step runs in k_resident.  A c2 step (3 particles
-// a cell) takes, there and as a chain of kernels (us): 1,000 particles 10.2 /
-// 21.1, 100,000 22.9 / 27.0, 300,000 32.0 / 32.5, 600,000 40.6 / 40.1, 1M
-// 51.5 / 48.8, 1.2M 56.4 / 52.1.  c3 the same within 1.
+// Cells up to which a binned step may run in k_resident (its particles are
+// limited too, see resident()).
 constexpr uint32_t kResidentCells = 150000;
 // Mean zeroth-order births per step that one CTA counts and bins beside the
 // others' records (k_resident, k_bin); more are counted by k_zeroth and dealt
@@ -183,10 +181,24 @@ struct bd_system {
   // The binned step of a small system runs in k_resident: no panels (their
   // walk needs more registers than the resident phases have), few births a
   // step (one CTA makes them), and small enough that launches and latency
-  // outweigh the work.
-  double births = 0.0;  // mean zeroth-order births per step
+  // outweigh the work on the quarter of the SMs that it takes (it holds them
+  // for many steps; the rest is for other handles' streams).  A c2 step (3
+  // particles a cell), there and as a chain of kernels, us: 4,001 particles
+  // 10.9 / 21.2, 20,000 14.7 / 24.6, 40,000 20.3 / 25.9, 60,000 23.2 / 26.4,
+  // 80,000 27.5 / 27.3, 100,000 32.1 / 27.7; 100,000 at 8 a cell 32 / 39, at 20
+  // 47 / 79, at 60 316 / 958; with many candidate pairs (500 particles per unit
+  // volume, 3 a cell) 40,000 53 / 56, 60,000 66 / 59.  Where cells of more than
+  // 128 particles are the rule the chain's large-cell kernel has the whole grid
+  // (20,000 at 150 a cell: 167 / 94).  Sparse grids, of at most 1.5 particles a
+  // cell, stay in it up to kResidentCells; the chain is the faster there above
+  // 10,000 particles (100,000 in 148,877 cells 37 / 27, 200,000 on half of the
+  // SMs 39 / 32).
+  double births = 0.0;   // mean zeroth-order births per step
+  uint64_t planned = 0;  // particles the instances were laid out for
   bool resident() const {
-    return binned && panels.empty() && n_cells <= kResidentCells && births <= kFewBirths && shape.grid_resident > 0;
+    return binned && panels.empty() && n_cells <= kResidentCells && births <= kFewBirths && shape.grid_resident > 0 &&
+           planned <= (uint64_t)kBigCell * n_cells &&
+           ((n_cells <= kResidentDense && planned <= kResidentParticles) || 2 * planned <= 3ull * n_cells);
   }
   Path path() const {
     return diffuse_only() ? Path::kDiffuseOnly
@@ -599,9 +611,12 @@ bd_status layout_cells(bd_system* h) {
   h->n_cells = (uint32_t)base;
   h->n_tiles = (uint32_t)((base + kScanTile - 1) / kScanTile);
   h->births = 0.0;
+  h->planned = 0;
   for (int k = 0; k < I; k++)
-    if (!h->server || h->slot_used[k])
+    if (!h->server || h->slot_used[k]) {
       for (int z : h->zero_list) h->births += h->derived[k].rx[z].prob;
+      if (k < (int)h->plan_n.size()) h->planned += h->plan_n[k];
+    }
   if (h->host_only) return BD_OK;
   // grow-only: a serving handle lays its cells out again at every admission,
   // and cudaFree would wait for the whole device

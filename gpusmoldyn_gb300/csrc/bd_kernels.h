@@ -97,8 +97,16 @@ int match_grid(int n_sm);
 int scan_grid(int n_sm);
 // CTAs of the large-cell kernel: at most 304, all resident on n_sm SMs.
 int big_grid(int n_sm);
-// CTAs of 1024 threads, at most one per SM, that k_resident can keep resident on n_sm SMs.
+// CTAs of 1024 threads, at most one per SM, that k_resident can keep resident
+// on n_sm SMs (0: too few SMs for it).
 int resident_grid(int n_sm);
+// Cells with more records than this are handed from k_pairs_cells to
+// k_pairs_big, which spreads their records over the whole grid.
+constexpr uint32_t kBigCell = 128;
+// Cells and particles up to which a system of more than 1.5 particles a cell
+// runs in k_resident, on a quarter of the SMs; particles up to which a sparser
+// one takes a quarter (else half).
+constexpr uint32_t kResidentDense = 18000, kResidentParticles = 100000, kResidentSparse = 80000;
 // Most steps of one launch of k_resident: long enough to hide the launch,
 // short enough to let other streams in.  Most reactions of its one-instance
 // variant.

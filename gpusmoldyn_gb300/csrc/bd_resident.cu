@@ -6,8 +6,10 @@
 // the whole step runs in one cooperative kernel that stays resident for many
 // steps, and what bounds it is round trips to L2 (0.4 us each): a barrier of
 // the grid is three of them.  c2 steps, chain and here, us: 1,000 particles
-// 21.1 / 10.2, 40,000 25.8 / 16.5, 100,000 27.0 / 22.9, 300,000 32.5 / 32.0;
-// above that the chain is faster.  So a step has as few barriers as it can:
+// 21.9 / 11.0, 10,000 22.7 / 12.7, 40,000 25.9 / 20.3, 80,000 27.3 / 27.5, on at
+// most a quarter of the SMs (on all of them 17.0 at 40,000 and 23.6 at 100,000,
+// but then nothing else runs beside it); 100,000 at 8 a cell 38.8 / 32.4, at 20
+// 78.6 / 46.7, where the chain's warps take turns of 32 cells.  So a step has as few barriers as it can:
 // two when it has no candidate pairs.
 //   * The cell scan is not a phase: after binning every CTA scans all counts
 //     for itself into shared memory (up to kSmallCells cells; above that the
@@ -35,7 +37,7 @@
 namespace bd {
 namespace {
 
-// CTAs of 1024 threads, at most one per SM: a barrier of 608 CTAs of 256
+// CTAs of 1024 threads, one per SM: a barrier of 608 CTAs of 256
 // threads took about twice the time of one of 152.
 constexpr int kThreads = 1024, kWarps = kThreads / 32;
 // Cells whose starts every CTA keeps in shared memory (128 KiB beside the
@@ -150,7 +152,8 @@ __device__ __forceinline__ uint32_t scan_counts(const uint32_t* counts, uint32_t
 }
 
 // The parts that few steps reach, or that one CTA runs, are calls: inlined,
-// their registers made the two streaming phases spill.
+// their registers made the streaming phases spill more.  (At the 64 registers
+// of 1,024 threads every variant spills some: 216 to 328 bytes of stores.)
 template <bool kHasBim>
 __device__ __noinline__ bool big_cells(const KParams& p, DevCtrl* c, unsigned long long* s_key) {
   const unsigned long long queued = __ldcg(&c->big_queue);
@@ -372,16 +375,25 @@ int resident_grid(int n_sm) {
                           resident_ctas<true, false, true>(), resident_ctas<true, false, false>(),
                           resident_ctas<false, true, true>(), resident_ctas<false, true, false>(),
                           resident_ctas<false, false, true>(), resident_ctas<false, false, false>()});
-  return std::min(a * n_sm, 255);  // the arrival word's failure field
+  const int grid = std::min(a * n_sm, 255);  // the arrival word's failure field
+  // a quarter of them has to hold the starts of the largest grid (150,000
+  // cells) between them
+  return grid / 4 < 5 ? 0 : grid;
 }
 
 void enqueue_resident(const KParams& p, bool table, bool has_bim, uint32_t nsteps, uint64_t n_slots,
                       const LaunchShape& shape, cudaStream_t s) {
   // 8 warps of records per CTA while there are SMs for it: fewer CTAs meet
   // sooner, more SMs work faster.  A CTA's range of cells has to fit its
-  // shared memory (kSmallCells) however few the records.
+  // shared memory (kSmallCells) however few the records.  A quarter of the SMs
+  // at most, half for larger sparse grids: a launch holds its SMs for
+  // up to 64 steps, and with all of them other streams' work waited for it.
+  // Handles of 40,000 particles side by side, us a step of each, all SMs /
+  // a quarter / the chain of kernels: one 17 / 20 / 26, two 33 / 21 / 30, four
+  // 65 / 21 / 35, eight 130 / 41 / 50, sixteen - / 82 / 98.
   const uint64_t want = std::max<uint64_t>({(n_slots + 255u) / 256u, (p.n_cells + 4095u) / 4096u, 1u});
-  const unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)std::max(shape.grid_resident, 1));
+  const int share = p.n_cells <= kResidentDense || n_slots <= kResidentSparse ? 4 : 2;
+  const unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)std::max(shape.grid_resident / share, 1));
   const bool single = p.n_inst == 1 && p.S <= kCtxSpecies && p.U <= kCtxUni && p.R <= kResidentReactions;
 #define BD_RESIDENT(T, B, S) launch<T, B, S>(p, nsteps, grid, s)
   if (table) {

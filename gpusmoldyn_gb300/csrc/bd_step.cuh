@@ -659,9 +659,6 @@ __device__ __forceinline__ void emit_pair(const KParams& p, DevCtrl* c, const ui
   else raise(c, kStatPairs);
 }
 
-// Cells with more records than this are handed from k_pairs_cells to
-// k_pairs_big, which gives each of them a whole CTA.
-constexpr uint32_t kBigCell = 128;
 constexpr uint32_t kBigChunk = 2048;  // records of a unit: sorted in one pass through shared memory (16 KiB of keys)
 constexpr int kBigGrid = 304;  // most CTAs of the large-cell kernel (cells they take in turn)
 

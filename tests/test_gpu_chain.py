@@ -51,3 +51,19 @@ def test_large_cells_without_second_order_reactions(n, sort):
     assert s.kernels_per_step() > 1
     run_parity(s, 2)
     s.close()
+
+
+@pytest.mark.parametrize("n,cells,kernels", [
+    (50000, 26, 1),       # 17,576 cells
+    (50000, 27, 5),       # 19,683
+    (100000, 26, 1),      # the most particles
+    (100001, 26, 5),
+    (60000, 35, 1),       # 42,875 cells: 1.4 a cell
+    (3456, 3, 1),         # 128 a cell
+    (3457, 3, 5),         # and one more: large cells are the rule
+], ids=lambda v: str(v))
+def test_the_line_between_k_resident_and_the_chain(n, cells, kernels):
+    s = system(n, cells, kon=0.2)
+    assert s.kernels_per_step() == kernels
+    run_parity(s, 4, batch=2)
+    s.close()
