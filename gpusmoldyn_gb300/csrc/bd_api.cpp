@@ -36,9 +36,14 @@ constexpr int kGraphBatch = 16;
 // limited too, see resident()).
 constexpr uint32_t kResidentCells = 150000;
 // Mean zeroth-order births per step that one CTA counts and bins beside the
-// others' records (k_resident, k_bin); more are counted by k_zeroth and dealt
-// out over the grid.
-constexpr double kFewBirths = 4096.0;
+// others' records; more are counted by k_zeroth and dealt out over the grid.
+// By the last CTA of k_bin / by k_zeroth and the grid, us a step: 100,000
+// particles, 1,000 births 32.5 / 30.6, 4,000 46.5 / 32.9 (38.8 before k_bin made
+// births); 1M particles, 1,000 births 49.2 / 46.4, 4,000 63.5 / 49.3 (61.1); 16M
+// c3 particles 4 us less by the CTA, whose births hide behind the records.  In
+// k_resident, whose alternative is the chain, 30,000 particles, 4,000 births:
+// 28.5 / 31.8.
+constexpr double kFewBirths = 1000.0, kResidentBirths = 4096.0;
 // Largest bin array the automatic sort mode accepts.
 constexpr uint64_t kBinBudgetBytes = 32ull << 30;
 
@@ -196,9 +201,10 @@ struct bd_system {
   double births = 0.0;   // mean zeroth-order births per step
   uint64_t planned = 0;  // particles the instances were laid out for
   bool resident() const {
-    return binned && panels.empty() && n_cells <= kResidentCells && births <= kFewBirths && shape.grid_resident > 0 &&
+    return binned && panels.empty() && n_cells <= kResidentCells && shape.grid_resident > 0 &&
            planned <= (uint64_t)kBigCell * n_cells &&
-           ((n_cells <= kResidentDense && planned <= kResidentParticles) || 2 * planned <= 3ull * n_cells);
+           ((n_cells <= kResidentDense && planned <= kResidentParticles && births <= kResidentBirths) ||
+            (2 * planned <= 3ull * n_cells && births <= kFewBirths));
   }
   Path path() const {
     return diffuse_only() ? Path::kDiffuseOnly

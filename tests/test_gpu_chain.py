@@ -16,16 +16,17 @@ pytestmark = pytest.mark.gpu
 CELLS = 54  # 157,464 cells of edge 0.25
 
 
-@pytest.mark.parametrize("births", [0.7, 40.0, 2000.0])
-def test_bins_overflow_beside_births_in_the_last_cta(births):
+@pytest.mark.parametrize("births,kernels", [(0.7, 5), (40.0, 5), (499.0, 5), (501.0, 6), (2000.0, 6)])
+def test_bins_overflow_beside_births(births, kernels):
     """A cluster overflows its bin while the last CTA of k_bin makes the
-    step's births: the step stops whole and is replayed with larger bins."""
+    step's births (1,000 by two reactions at most; more are k_zeroth's): the
+    step stops whole and is replayed with larger bins."""
     s = system(3000, CELLS, births=births)
     g = rng(17)
     pos = uniform_positions(g, 3000, (0, 0, 0), (0.25 * CELLS,) * 3)
     pos[:400] = uniform_positions(g, 400, (0.3,) * 3, (0.4,) * 3)
     s.set_particles(pos, (np.arange(3000) % 3).astype(np.int32))
-    assert s.kernels_per_step() == 5  # no k_zeroth: the births are k_bin's
+    assert s.kernels_per_step() == kernels
     run_parity(s, 6, batch=3)
     s.close()
 
