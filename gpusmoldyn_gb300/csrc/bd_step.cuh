@@ -1240,6 +1240,41 @@ __device__ __forceinline__ uint32_t runs_rank(const float4* v, uint32_t w, uint3
   return rank;
 }
 
+// Bitonic network over the keys s_key[0, size), size a power of two, by the
+// threads of the CTA.
+template <class Less>
+__device__ __forceinline__ void bitonic_network(unsigned long long* s_key, uint32_t size, Less&& less) {
+  for (uint32_t k = 2; k <= size; k <<= 1) {
+    for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+      for (uint32_t t = threadIdx.x; t < size / 2; t += blockDim.x) {
+        const uint32_t i = ((t & ~(j - 1u)) << 1) | (t & (j - 1u)), ixj = i | j;
+        const unsigned long long q0 = s_key[i], q1 = s_key[ixj];
+        const bool swap = less(q1, q0) == ((i & k) == 0);
+        s_key[i] = swap ? q1 : q0;
+        s_key[ixj] = swap ? q0 : q1;
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// Records of a unit with the same x bits are put in order by counting over
+// their stretch of equal keys, up to this many apart; a unit with a longer
+// stretch goes through the network once more, by all four words (by index
+// when identical).  2,000 immobile molecules with one x: 845 us a step when
+// the stretch was counted over whatever its length, 82 so, 38 with distinct x
+// (and 89 with a network over whole records, one CTA a cell).
+constexpr uint32_t kTieStretch = 8;
+__device__ __noinline__ void sort_tied_keys(unsigned long long* s_key, uint32_t size, uint32_t len, const CellView cb,
+                                            uint32_t first) {
+  bitonic_network(s_key, size, [&](unsigned long long a, unsigned long long b) {
+    const uint32_t i = (uint32_t)a, j = (uint32_t)b;
+    if (a >> 32 != b >> 32 || i >= len || j >= len) return a < b;  // past the unit: all ones
+    const float4 q = cb[first + i], r = cb[first + j];
+    return rec_less(q, r) || (i < j && rec_equal(q, r));
+  });
+}
+
 // Canonical order of the queued cells.  Phase 1 sorts each unit in shared
 // memory (a bitonic network over keys) into big_scratch;
 // then each merge pass joins up to kBigWays runs into one: a record's place
@@ -1271,18 +1306,14 @@ __device__ bool big_sort(const KParams& p, DevCtrl* c, uint32_t nbig, uint32_t u
     for (uint32_t i = threadIdx.x; i < size; i += blockDim.x)
       s_key[i] = i < len ? (unsigned long long)__float_as_uint(cb[b.first + i].x) << 32 | i : ~0ull;
     __syncthreads();
-    for (uint32_t k = 2; k <= size; k <<= 1) {
-      for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-        for (uint32_t t = threadIdx.x; t < size / 2; t += blockDim.x) {
-          const uint32_t i = ((t & ~(j - 1u)) << 1) | (t & (j - 1u)), ixj = i | j;
-          const unsigned long long q0 = s_key[i], q1 = s_key[ixj];
-          const bool swap = (q1 < q0) == ((i & k) == 0);
-          s_key[i] = swap ? q1 : q0;
-          s_key[ixj] = swap ? q0 : q1;
-        }
-        __syncthreads();
-      }
-    }
+    bitonic_network(s_key, size, [](unsigned long long a, unsigned long long b) { return a < b; });
+    // molecules lined up in x (a lattice, a membrane, a release that does not
+    // diffuse): stretches of equal keys too long to count over
+    bool tied = false;
+    for (uint32_t i = threadIdx.x; i + kTieStretch < len; i += blockDim.x)
+      tied |= s_key[i] >> 32 == s_key[i + kTieStretch] >> 32;
+    tied = __syncthreads_or(tied) != 0;
+    if (tied) sort_tied_keys(s_key, size, len, cb, b.first);
     const bool done = b.n <= kBigChunk;
     float4* tmp = big_buffer(p, b.cs, 0) + b.first;
     for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) {
@@ -1292,8 +1323,8 @@ __device__ bool big_sort(const KParams& p, DevCtrl* c, uint32_t nbig, uint32_t u
       // when identical), counted over their stretch of equal keys
       uint32_t at = i, lo = i, hi = i + 1u;
       const uint32_t xb = (uint32_t)(key >> 32);
-      while (lo > 0 && (uint32_t)(s_key[lo - 1u] >> 32) == xb) --lo;
-      while (hi < len && (uint32_t)(s_key[hi] >> 32) == xb) ++hi;
+      while (!tied && lo > 0 && (uint32_t)(s_key[lo - 1u] >> 32) == xb) --lo;
+      while (!tied && hi < len && (uint32_t)(s_key[hi] >> 32) == xb) ++hi;
       if (hi - lo > 1u) {
         at = lo;
         for (uint32_t m = lo; m < hi; ++m) {
