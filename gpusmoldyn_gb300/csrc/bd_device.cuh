@@ -5,8 +5,8 @@
 // __fmul_rn, __fadd_rn, __fsqrt_rn), so the compiler cannot contract or
 // reorder it and a CPU program that performs the same IEEE operations gets
 // the same bits.  Only the production normal generator (Box-Muller with
-// the hardware approximations __logf / __sincosf) is not bit-reproducible
-// on a CPU; the table mode is.
+// the hardware approximations of box_muller_radius and __sincosf) is not
+// bit-reproducible on a CPU; the table mode is.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -101,21 +101,23 @@ __device__ __forceinline__ double u53_to_unit(uint32_t a, uint32_t b) {
   return (double)m * 1.1102230246251565e-16;
 }
 
-// log and 1 / sqrt of a normal number by the hardware's approximations.  The
-// bits are those of __logf and rsqrtf (compared for every 24-bit uniform and
-// the radii they give), without the instructions that scale a subnormal
-// argument, which a uniform of 2^-25 or more and a radius of 1e-30 or more
-// never are.
-__device__ __forceinline__ float log_normal(float x) {
-  float y;
-  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return 0.69314718055994531f * y;
+// The Box-Muller radius sqrt(-2 ln a) of a uniform a in [2^-25, 1]:
+// q = -2 ln a = -2 ln 2 log2 a, and sqrt(q) = q / sqrt(q), by the base-2
+// logarithm and the reciprocal square root that the PTX ISA documents as
+// approximations: lg2.approx errs by at most 2^-22, absolutely between 1/2 and
+// 2 and relatively elsewhere, rsqrt.approx by 2^-22.9 relatively.  Neither a
+// nor q is ever subnormal (the logarithm may come out as 0 at a = 1, and the
+// radius stays finite).
+__device__ __forceinline__ float box_muller_radius(float a) {
+  float lg, rs;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(lg) : "f"(a));
+  const float q = fmaxf(-1.3862943611198906f * lg, 1e-30f);
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(q));
+  return q * rs;
 }
-__device__ __forceinline__ float rsqrt_normal(float x) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
+
+// The uniform of a radius: never 0.
+__device__ __forceinline__ float radius_uniform(uint32_t v) { return u24_to_unit(v) + 2.98023223876953125e-08f; }
 
 // Three standard normals from words x, y, z of one Philox block; word w is
 // left for the first first-order coin.
@@ -134,12 +136,8 @@ __device__ __forceinline__ void normals3(const U4& r, const float* __restrict__ 
   } else {
     // hardware approximations (MUFU lg2 / rsqrt / sin / cos): absolute
     // errors ~1e-6, far below the statistical resolution of the step
-    const float a = u24_to_unit(r.x) + 2.98023223876953125e-08f;  // (0, 1)
-    const float c = u24_to_unit(r.z) + 2.98023223876953125e-08f;
-    // the log may round to 0 just below 1: keep the radius finite (0)
-    const float la = fmaxf(-2.0f * log_normal(a), 1e-30f), lc = fmaxf(-2.0f * log_normal(c), 1e-30f);
-    const float ra = la * rsqrt_normal(la);
-    const float rc = lc * rsqrt_normal(lc);
+    const float ra = box_muller_radius(radius_uniform(r.x));
+    const float rc = box_muller_radius(radius_uniform(r.z));
     float sa, ca, sc, cc;
     __sincosf(6.2831853071795865f * u24_to_unit(r.y), &sa, &ca);
     const uint32_t low = ((r.x & 0xFFu) << 24) | ((r.y & 0xFFu) << 16) | ((r.z & 0xFFu) << 8);
