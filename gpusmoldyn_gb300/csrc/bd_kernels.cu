@@ -882,9 +882,13 @@ void enqueue_diffuse(const KParams& p, bool table, uint32_t nsteps, uint64_t n_s
   // records, since the last round of a wave runs half empty.  One wave and a
   // CTA per 256 records, us: 1M records 1 step 17 / 51, 8 steps 43 / 59, 16
   // steps 75 / 77, 25 steps 111 / 107; 4M 34 / 182, 140 / 204, 262 / 271,
-  // 406 / 384.
+  // 406 / 384.  With little work in all the wave itself has fewer CTAs, since
+  // they count themselves on one word: 300,000 records, 1 step, three / eight
+  // per SM 10.4 / 16.7 (12.6 as k_diffuse and k_finalize_inplace), 1M 1 step
+  // 14.9 / 17.6, 4 steps 27.6 / 28.2; 4M, 4 steps 83 / 78.
   const uint64_t ctas = std::max<uint64_t>((n_slots + 255u) / 256u, 1u);
-  const unsigned grid = (unsigned)std::min<uint64_t>(ctas, nsteps < 20u ? 152u * kDiffuseCtas : 1u << 20);
+  const unsigned wave = 152u * (n_slots * nsteps <= 4000000u ? 3u : kDiffuseCtas);
+  const unsigned grid = (unsigned)std::min<uint64_t>(ctas, nsteps < 20u ? wave : 1u << 20);
   if (table) k_diffuse_steps<true><<<grid, 256, 0, s>>>(p, nsteps);
   else k_diffuse_steps<false><<<grid, 256, 0, s>>>(p, nsteps);
 }
