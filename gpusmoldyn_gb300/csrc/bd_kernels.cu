@@ -261,8 +261,9 @@ __device__ __noinline__ void bin_births(const KParams& p, DevCtrl* c, const Sing
   }
 }
 
-// Bound by issue (58% of the slots) and the latency of its loads and atomics
-// at 32 warps per SM; what it does per record is what it costs.  16M c3 step:
+// Bound by its stores, 16 bytes each into sectors that stay partly empty (a
+// bare kernel with the same copy, atomics and stores takes 188 us at 16M, 106
+// when it only copies and counts); the issue slots are half busy.  16M c3 step:
 // 227 us -> 202 by taking out of the record's path what rarely applies (the
 // first-order loop behind a bound on the coin's word, one in-box test for the
 // three axes, no lower cell bound, births) and what can be laid out (Philox
@@ -308,8 +309,8 @@ __global__ void __launch_bounds__(256, kMinBlocks) k_bin(const __grid_constant__
 // is empty: a warp of slow walks does not hold the others' share.  Bound by
 // the latency of its load chains.  c3 in a cell, 2M / 16M particles: 84 / 102
 // us before the finer panel grid and the panel heads in one load; then 39 /
-// 66 us at four CTAs per SM (64 registers, spills), 36 / 60 at three, 36 / 65
-// at two.
+// 66 us at four CTAs per SM (64 registers, 92 to 144 bytes of spills), 36 / 60
+// at three (80 registers, 16 to 72 bytes), 36 / 65 at two.
 template <bool kTable, bool kSingle>
 __global__ void __launch_bounds__(256, 3) k_bin_surface(KParams p) {
   __shared__ DevSpecies s_species[kSingle ? kCtxSpecies : 1];

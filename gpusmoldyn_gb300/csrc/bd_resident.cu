@@ -153,7 +153,7 @@ __device__ __forceinline__ uint32_t scan_counts(const uint32_t* counts, uint32_t
 
 // The parts that few steps reach, or that one CTA runs, are calls: inlined,
 // their registers made the streaming phases spill more.  (At the 64 registers
-// of 1,024 threads every variant spills some: 216 to 328 bytes of stores.)
+// of 1,024 threads every variant spills some: 204 to 328 bytes of stores.)
 template <bool kHasBim>
 __device__ __noinline__ bool big_cells(const KParams& p, DevCtrl* c, unsigned long long* s_key) {
   const unsigned long long queued = __ldcg(&c->big_queue);

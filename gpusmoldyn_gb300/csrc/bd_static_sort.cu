@@ -42,7 +42,7 @@ constexpr uint32_t kStaticMaxTiles = kStaticMaxCells / kStaticTile;
 constexpr uint32_t kCtrlWords = 2;  // crowded-cell count, crowded-cell ticket
 constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr int kMaxDevices = 64;
-constexpr uint32_t kThreadCell = 32;    // largest cell ordered by a single thread
+constexpr uint32_t kThreadCell = 32;    // largest cell ordered by a row of lanes
 constexpr uint32_t kChunk = 2048;       // records a block orders in shared memory (32 KiB)
 constexpr int kCrowdThreads = 512;
 
